@@ -23,6 +23,7 @@ struct dpack_tables
   std::shared_ptr<const encode_plan> plan;  // (kept alive: the key is its identity)
   std::vector<std::vector<int>> nexps;
   std::vector<unsigned> bricks_per_chunk;
+  dtype type = dtype::float32;  // (raw exponents are a byte or two wide)
   dpack_plan P;
   std::vector<int4> subs;
   std::vector<int> seg_sub0;
@@ -46,13 +47,14 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
     nexps[l] = levels[l].nexps;
   std::vector<unsigned> bpc(f.bricks_per_chunk.begin(), f.bricks_per_chunk.end());
   std::shared_ptr<dpack_tables> T = std::static_pointer_cast<dpack_tables>(ctx->dpack);
-  if (!T || T->plan != plan || T->nexps != nexps || T->bricks_per_chunk != bpc)
+  if (!T || T->plan != plan || T->nexps != nexps || T->bricks_per_chunk != bpc || T->type != f.type)
   {
     ctx->dpack.reset();
     T = std::make_shared<dpack_tables>();
     T->plan = plan;
     T->nexps = nexps;
     T->bricks_per_chunk = bpc;
+    T->type = f.type;
     int e = dpack_make_plan(f, *plan, nexps, &T->P);
     if (e)
       return e;

@@ -106,3 +106,18 @@ def test_repeated_encodes_with_premapped_files_equal_fresh_encodes(tmp_path):
     assert big >= 64 << 20  # (files from 64 MB on are allocated ahead)
     for got, want in (("a1", "fa"), ("a2", "fa"), ("b1", "fb"), ("c1", "fc")):
         assert compare_dirs(os.path.join(out, want, "rp"), os.path.join(out, got, "rp")) == [], got
+
+
+@pytest.mark.gpu
+def test_sample_type_changes_between_encodes_of_one_shape(idx2g, tmp_path):
+    """A float32 and then a float64 field of one shape: the second encode packs its own (wider)
+    exponents, so its files equal those of an encode that never saw the first field."""
+    from idx2_b200.synthetic import grf_field
+    f = grf_field(70, 66, 65, seed=3, scale="unit")
+    files = []
+    for name, first in (("a", "float32"), ("b", "float64")):
+        for dt in (first, "float64"):
+            idx2g.encode(f.astype(dt), out_dir=str(tmp_path / name), name="t", field_name="f", num_levels=2,
+                         tolerance=1e-3)
+        files.append({p.name: p.read_bytes() for p in sorted((tmp_path / name).rglob("*.bin"))})
+    assert files[0] == files[1] and files[0]
