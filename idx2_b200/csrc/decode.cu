@@ -28,6 +28,7 @@ namespace
 {
 
 #include "decode_kernel.cuh"
+#include "decode_bricks.cuh"
 
 } // namespace
 
@@ -718,11 +719,16 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
     return OutOfMemory;
   // the plane-table path's shared memory (float staging rows for a float32 output), and the
   // three-CTA build for an output level of many bricks with a float32 output
-  const size_t smem = dec_smem_bytes(true, r0.f32);
+  // 3D bricks of one plane per key: k_decode_bricks (its header has both sides' times). Its
+  // registers hold one 4^3 block per lane, so 2D bricks, whose blocks are 4 x 4, keep
+  // k_decode_level, as do several planes per key (other tables) and the coefficient mode.
+  const bool by_lane = !r0.is2d && r0.bpc == 1 && !coeff_out;
+  const size_t smem = by_lane ? sizeof(brick_smem) : dec_smem_bytes(true, r0.f32);
+  cudaFuncSetAttribute(k_decode_bricks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem));
   cudaFuncSetAttribute(k_decode_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
   cudaFuncSetAttribute(k_decode_level<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
   int occ3 = 0;
-  if (r0.f32 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_decode_level<3>, kThreads, smem) != cudaSuccess)
+  if (!by_lane && r0.f32 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_decode_level<3>, kThreads, smem) != cudaSuccess)
   {
     cudaGetLastError();
     occ3 = 0;
@@ -743,6 +749,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
     if (keep)
     {
       keep->bricks.assign((size_t)L, nullptr);
+      keep->natural = by_lane;
       keep->sig.assign((size_t)L, std::vector<int>());
     }
     size_t nev = 0;  // levels timed (event pairs of the pool)
@@ -832,7 +839,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       three = three && occ3 >= 3 && nbr >= 6 * ctx->num_sms;
       const int cps = three ? 3 : 2;
       int grid = nbr < cps * ctx->num_sms ? nbr : cps * ctx->num_sms;
-      double* d_slots = (double*)ctx->ws("dec.slots", (size_t)grid * (size_t)NB * 8);
+      double* d_slots = (double*)ctx->ws("dec.slots", (size_t)grid * (size_t)(by_lane ? kSlotBrick : NB) * 8);
       if (!d_bricks || !d_reqs || (nstore && !d_level) || !d_slots)
         return OutOfMemory;
       // the level's tables through pinned staging of its own (copies stay asynchronous; the
@@ -986,7 +993,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
           ag.nbricks = cuts[g + 1] - cuts[g];
           ag.unit_off = d_uoff + (size_t)cuts[g] * (size_t)r0.nsb;
           const int gg = ag.nbricks < grid ? ag.nbricks : grid;
-          (three ? k_decode_level<3> : k_decode_level<2>)<<<gg, kThreads, smem, st>>>(ag);
+          (by_lane ? k_decode_bricks : three ? k_decode_level<3> : k_decode_level<2>)<<<gg, kThreads, smem, st>>>(ag);
           ++ctx->launches;
           const size_t z_next =
             g + 2 < cuts.size() ? (size_t)hb[(size_t)cuts[g + 1]].dst_from[2] : (size_t)r0.out_dims.z;
@@ -1006,7 +1013,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       }
       else
       {
-        (three ? k_decode_level<3> : k_decode_level<2>)<<<grid, kThreads, smem, st>>>(a);
+        (by_lane ? k_decode_bricks : three ? k_decode_level<3> : k_decode_level<2>)<<<grid, kThreads, smem, st>>>(a);
         ctx->launches += 3;
       }
       cudaEventRecord(t1, st);
@@ -1060,8 +1067,9 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
 namespace
 {
 
-// Pieces of kept bricks (subband-major) to a dense buffer, x fastest: a CTA per piece.
-__global__ void k_gather_pieces(const brick_piece* pieces, int n, int is2d, double* out)
+// Pieces of kept bricks (subband-major, or natural order) to a dense buffer, x fastest: a CTA per
+// piece.
+__global__ void k_gather_pieces(const brick_piece* pieces, int n, int is2d, int natural, double* out)
 {
   for (int pi = blockIdx.x; pi < n; pi += gridDim.x)
   {
@@ -1071,15 +1079,16 @@ __global__ void k_gather_pieces(const brick_piece* pieces, int n, int is2d, doub
     for (int i = threadIdx.x; i < cnt; i += blockDim.x)
     {
       const int x = i % p.dims[0], y = (i / p.dims[0]) % p.dims[1], z = i / nxy;
-      out[p.out + i] = p.src[sbm(p.from[0] + x, p.from[1] + y, p.from[2] + z, is2d)];
+      const int bx = p.from[0] + x, by = p.from[1] + y, bz = p.from[2] + z;
+      out[p.out + i] = p.src[natural ? (bz * 33 + by) * 33 + bx : sbm(bx, by, bz, is2d)];
     }
   }
 }
 
 } // namespace
 
-int decode_device::gather_bricks(device_ctx* ctx, const std::vector<brick_piece>& pieces, bool is2d, size_t total,
-                                 double* host_out)
+int decode_device::gather_bricks(device_ctx* ctx, const std::vector<brick_piece>& pieces, bool is2d, bool natural,
+                                 size_t total, double* host_out)
 {
   if (pieces.empty() || total == 0)
     return NoError;
@@ -1091,7 +1100,8 @@ int decode_device::gather_bricks(device_ctx* ctx, const std::vector<brick_piece>
     return OutOfMemory;
   cudaMemcpyAsync(d_p, pieces.data(), sizeof(brick_piece) * pieces.size(), cudaMemcpyHostToDevice, st);
   const int n = (int)pieces.size();
-  k_gather_pieces<<<n < 8 * ctx->num_sms ? n : 8 * ctx->num_sms, 256, 0, st>>>(d_p, n, is2d ? 1 : 0, d_out);
+  k_gather_pieces<<<n < 8 * ctx->num_sms ? n : 8 * ctx->num_sms, 256, 0, st>>>(d_p, n, is2d ? 1 : 0,
+                                                                             natural ? 1 : 0, d_out);
   ++ctx->launches;
   if (cudaGetLastError() != cudaSuccess)
     return CudaError;

@@ -25,6 +25,11 @@
 //    or fewer) are rebuilt first, into three 33 x 33 faces in shared memory.
 //
 // Kept bricks are stored x fastest, 33^3 doubles, in natural order.
+//
+// Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
+// 7.4 ms against 28.3 ms with k_decode_level; one brick per CTA (8 bricks) 59 against 184 us. At
+// 512^3 57 K warp instructions per brick (354 K before), 26% issue activity: what is left is the
+// latency of the L2 round trips at 16 warps per SM (128 registers a thread).
 #pragma once
 
 constexpr int kFaceRow = 33;

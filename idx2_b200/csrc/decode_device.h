@@ -60,12 +60,13 @@ struct decode_request
 };
 
 // Brick-map mode (the reference's HashMap output, Core/idx2Decode.cpp:446-477): every decoded
-// level's bricks are kept on the device (subband-major, in plan order) with a significance flag
-// per brick (a block of a subband > 0, or of the coarsest level, was decoded).
+// level's bricks are kept on the device (x fastest where `natural`, else subband-major; in plan
+// order) with a significance flag per brick (a block of a subband > 0, or of the coarsest level, was decoded).
 struct decode_keep
 {
   std::vector<const double*> bricks;     // per level l: [plan bricks][33^3] or null (not decoded)
   std::vector<std::vector<int>> sig;     // per level l: significance per plan brick
+  bool natural = false;
 };
 
 // A part of a kept brick copied out by gather_bricks: samples [from, from + dims) of the
@@ -113,9 +114,9 @@ public:
   int decode_batch(device_ctx* ctx, const std::vector<const decode_request*>& rqs, void* const* outs,
                    const size_t* out_bytes, bool out_on_device, double* kernel_ms, void* coeff_out = nullptr,
                    decode_keep* keep = nullptr);
-  // Copy pieces of kept bricks (subband-major) into a host buffer of `total` doubles.
-  static int gather_bricks(device_ctx* ctx, const std::vector<brick_piece>& pieces, bool is2d, size_t total,
-                           double* host_out);
+  // Copy pieces of kept bricks into a host buffer of `total` doubles.
+  static int gather_bricks(device_ctx* ctx, const std::vector<brick_piece>& pieces, bool is2d, bool natural,
+                           size_t total, double* host_out);
   // Allocation-free decode into a device buffer: every temporary lives in a fixed static
   // device array of decode.cu (limits and semantics there and in include/idx2g.h).
   int decode_noalloc(device_ctx* ctx, const decode_request& rq, void* d_out, size_t out_bytes,

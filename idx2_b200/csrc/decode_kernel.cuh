@@ -61,8 +61,15 @@ struct dec_args
   void* coeff_out;
   // decoded bit planes from k_decode_planes (null: the kernel runs the wavefront itself)
   const unsigned long long* planes;
-  const unsigned long long* unit_off;  // [brick][subband] byte offset of the unit's table, ~0: none
+  const unsigned long long* unit_off;  // [brick][subband] the unit's table (kUnitOffMask), ~0: none
 };
+
+// A unit's plane table. One plane per key: block b's planes from the top down are the first
+// words of its row b, rows of `stride` words (the most planes of a block of the unit, rounded up
+// to a pair, so that a row starts 16-byte aligned); unit_off holds the byte offset in the low 56
+// bits and the stride above. Several planes per key: rows by wavefront step (plane_wavefront).
+constexpr int kUnitStrideShift = 56;
+constexpr unsigned long long kUnitOffMask = (1ull << kUnitStrideShift) - 1ull;
 
 // Arguments of the bit-plane kernel (one warp per (brick, subband) unit).
 struct dec1_args
@@ -344,8 +351,9 @@ __device__ __forceinline__ void ilift33(double (&v)[33])
 // Bit planes of one (brick, subband): the wavefront of the group-test decoder alone
 // (Core/idx2Decode.cpp:141-202). Channel c = kmax - key is owned by lane c % 32 (G groups of
 // 32 channels); at step t it decodes its plane of block t - c, taking the block's significance
-// count from channel c - 1 at step t - 1. The plane masks of step t are stored as row t of the
-// unit's table (row length nkeys): block b's plane in channel c is row b + c, column c.
+// count from channel c - 1 at step t - 1. The plane masks go to the unit's table by block (see
+// kUnitOffMask); with several planes per key those of step t are row t of the table (row length
+// nkeys): block b's planes in channel c are row b + c, column c.
 // ---------------------------------------------------------------------------
 constexpr int kPlaneWarps = 8;
 
@@ -359,7 +367,7 @@ struct plane_smem
 template <int G, bool MULTI>
 __device__ __forceinline__ void plane_wavefront(const dec1_args& a, size_t fs, int nb, int nkeys, int kmax,
                                                 const int16_t* ktop, const uint8_t* npl, const uint8_t* nvl,
-                                                unsigned long long* T, int lane)
+                                                unsigned long long* T, int stride, int lane)
 {
   bit_reader rd[G];
   bool has[G];
@@ -429,10 +437,9 @@ __device__ __forceinline__ void plane_wavefront(const dec1_args& a, size_t fs, i
               X = decode_plane(rd[g], n, 1 << nvl[b]);
               n_out[g] = n;
             }
+            T[b * stride + top - key] = X;
           }
         }
-        if (c < nkeys)
-          T[(size_t)t * (size_t)nkeys + (size_t)c] = X;
       }
       else if (c < nkeys)
       {
@@ -470,7 +477,7 @@ __device__ __forceinline__ void plane_wavefront(const dec1_args& a, size_t fs, i
 // deferred to the second pass, or no room).
 struct plane_unit
 {
-  int run, nb, nkeys, kmax;
+  int run, nb, nkeys, kmax, stride;
   size_t fs;
   unsigned long long* T;
 };
@@ -481,7 +488,7 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, in
 {
   plane_unit u;
   u.run = 0;
-  u.nb = u.nkeys = u.kmax = 0;
+  u.nb = u.nkeys = u.kmax = u.stride = 0;
   u.fs = 0;
   u.T = nullptr;
   const int bi = unit / a.nsb, s = unit - bi * a.nsb;
@@ -494,7 +501,7 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, in
   }
   const int nb = a.nblocks[s];
   const size_t fs = (size_t)a.bricks[bi].flat * (size_t)a.nsb + (size_t)s;
-  int kmin = 1 << 30, kmax = -(1 << 30);
+  int kmin = 1 << 30, kmax = -(1 << 30), npmax = 0;
   for (int b = lane; b < nb; b += 32)
   {
     int d3[3], bd[3];
@@ -505,6 +512,7 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, in
     ktop[b] = (int16_t)top;
     npl[b] = (uint8_t)np;
     nvl[b] = (uint8_t)(2 * ((bd[0] > 1) + (bd[1] > 1) + (bd[2] > 1)));
+    npmax = np > npmax ? np : npmax;
     if (np)
     {
       if (top - np + 1 < 0)
@@ -540,8 +548,10 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, in
       a.wide_list[atomicAdd(a.wide_count, 1)] = unit;
     return u;
   }
+  const int stride = MULTI ? 0 : (__reduce_max_sync(0xffffffffu, npmax) + 1) & ~1;
   const unsigned long long bytes =
-    (unsigned long long)(nb + nkeys - 1) * (unsigned long long)nkeys * 8ull * (unsigned long long)a.bpc;
+    MULTI ? (unsigned long long)(nb + nkeys - 1) * (unsigned long long)nkeys * 8ull * (unsigned long long)a.bpc
+          : (unsigned long long)nb * (unsigned long long)stride * 8ull;
   unsigned long long base = 0;
   if (lane == 0)
     base = atomicAdd(a.cursor, bytes);
@@ -556,8 +566,9 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, in
     return u;
   }
   if (lane == 0)
-    a.unit_off[unit] = base;
+    a.unit_off[unit] = base | ((unsigned long long)stride << kUnitStrideShift);
   u.run = 1;
+  u.stride = stride;
   u.nb = nb;
   u.nkeys = nkeys;
   u.kmax = kmax;
@@ -596,7 +607,8 @@ __device__ __forceinline__ void plane_wavefront_pair(const dec1_args& a, const p
       }
     }
   }
-  const int my_steps = nb + nkeys - 1;
+  const int stride = U.stride;
+  unsigned long long* const T = U.T;
   const int sA = A.nb + A.nkeys - 1, sB = B.nb + B.nkeys - 1;
   const int steps = sA > sB ? sA : sB;
   int n_out = 0, stop_out = 0;
@@ -630,10 +642,9 @@ __device__ __forceinline__ void plane_wavefront_pair(const dec1_args& a, const p
           X = decode_plane(rd, n, 1 << nvl[b]);
           n_out = n;
         }
+        T[b * stride + top - key] = X;
       }
     }
-    if (c < nkeys && t < my_steps)
-      U.T[(size_t)t * (size_t)nkeys + (size_t)c] = X;
   }
 }
 
@@ -652,7 +663,7 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, WIDE ? 2 : (MULTI ? 6 : 4)) 
       const plane_unit A = prep_unit<false, false>(a, i, sm.ktop[warp][0], sm.np[warp][0], sm.nvl[warp][0], lane);
       plane_unit B;
       B.run = 0;
-      B.nb = B.nkeys = B.kmax = 0;
+      B.nb = B.nkeys = B.kmax = B.stride = 0;
       B.fs = 0;
       B.T = nullptr;
       if (i + 1 < nunits)
@@ -665,10 +676,10 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, WIDE ? 2 : (MULTI ? 6 : 4)) 
       {
         if (A.run)
           plane_wavefront<1, false>(a, A.fs, A.nb, A.nkeys, A.kmax, sm.ktop[warp][0], sm.np[warp][0],
-                                    sm.nvl[warp][0], A.T, lane);
+                                    sm.nvl[warp][0], A.T, A.stride, lane);
         if (B.run)
           plane_wavefront<1, false>(a, B.fs, B.nb, B.nkeys, B.kmax, sm.ktop[warp][1], sm.np[warp][1],
-                                    sm.nvl[warp][1], B.T, lane);
+                                    sm.nvl[warp][1], B.T, B.stride, lane);
       }
       __syncwarp();
     }
@@ -690,20 +701,20 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, WIDE ? 2 : (MULTI ? 6 : 4)) 
     {
       // several planes per key: units of up to 32 keys here, up to 64 in the second pass
       if (!WIDE)
-        plane_wavefront<1, true>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+        plane_wavefront<1, true>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
       else
-        plane_wavefront<2, true>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+        plane_wavefront<2, true>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     }
     else if (!WIDE)
-      plane_wavefront<1, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+      plane_wavefront<1, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     else if (nkeys <= 32)
-      plane_wavefront<1, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+      plane_wavefront<1, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     else if (nkeys <= 64)
-      plane_wavefront<2, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+      plane_wavefront<2, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     else if (nkeys <= 96)
-      plane_wavefront<3, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+      plane_wavefront<3, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     else
-      plane_wavefront<4, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, lane);
+      plane_wavefront<4, false>(a, fs, nb, nkeys, kmax, ktop, npl, nvl, T, U.stride, lane);
     __syncwarp();
   }
 }
@@ -860,7 +871,8 @@ __global__ void __launch_bounds__(kThreads, CPS) k_decode_level(const dec_args a
         const unsigned long long uo = a.unit_off[(size_t)bi * (size_t)a.nsb + (size_t)s];
         if (uo == ~0ull)
           continue;
-        const unsigned long long* T = a.planes + uo / 8;
+        const unsigned long long* T = a.planes + (uo & kUnitOffMask) / 8;
+        const int stride = (int)(uo >> kUnitStrideShift);
         const int nb = a.nblocks[s], nkeys = sm.nkeys[s], kmax = sm.kmax[s];
         const uint64_t* geom = a.geom + (size_t)s * kMaxBlocksPerSubband;
         int hx, hy, hz;
@@ -878,7 +890,6 @@ __global__ void __launch_bounds__(kThreads, CPS) k_decode_level(const dec_args a
         }
         const int dx = 17 - hx, dy = 17 - hy;
         double* const sbase = F + sbm_base(hx, hy, hz, a.is2d);
-        // plane k of block b (bit plane 63 - k) is in channel c0 + k, table row b + c0 + k;
         // blocks with nothing to decode (no planes, or not part of the request) stay zero
         auto load_planes = [&](int b, unsigned long long& x0, unsigned long long& x1) {
           x0 = 0;
@@ -891,12 +902,10 @@ __global__ void __launch_bounds__(kThreads, CPS) k_decode_level(const dec_args a
           const int top = sm.ktop[s][b], bpc = a.bpc;
           if (bpc == 1)
           {
-            // plane kk in channel c0 + kk, table row b + c0 + kk
-            const int c0 = kmax - top;
-            if (lane < np && c0 + lane < nkeys)
-              x0 = T[(size_t)(b + c0 + lane) * (size_t)nkeys + (size_t)(c0 + lane)];
-            if (lane + 32 < np && c0 + lane + 32 < nkeys)
-              x1 = T[(size_t)(b + c0 + lane + 32) * (size_t)nkeys + (size_t)(c0 + lane + 32)];
+            if (lane < np)
+              x0 = T[b * stride + lane];
+            if (lane + 32 < np)
+              x1 = T[b * stride + lane + 32];
             return;
           }
           // plane kk: channel c = kmax - key, step b + c, slot key * bpc + bpc - 1 - (top - kk)

@@ -912,7 +912,7 @@ int dataset_decode_brick_map(device_ctx* ctx, dataset_handle* h, const params& p
         dims_of.push_back(dims);
       }
   std::vector<double> samples((size_t)total);
-  e = decode_device::gather_bricks(ctx, pieces, is2d, (size_t)total, samples.data());
+  e = decode_device::gather_bricks(ctx, pieces, is2d, keep.natural, (size_t)total, samples.data());
   if (e)
     return e;
   FILE* fp = fopen(path, "wb");
