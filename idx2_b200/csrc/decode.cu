@@ -946,7 +946,9 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
         const int g1 = (p.unit_last - p.unit_first + kPlaneWarps - 1) / kPlaneWarps;
         if (r0.bpc == 1)
         {
-          k_decode_planes<false><<<(g1 + 1) / 2, kPlaneWarps * 32, 0, st>>>(p);  // two units per warp
+          // two units per warp where there are more of them than warps in flight
+          const int pair = p.unit_last - p.unit_first > 4 * kPlaneWarps * ctx->num_sms;
+          k_decode_planes_ring<<<pair ? (g1 + 1) / 2 : g1, kPlaneWarps * 32, 0, st>>>(p, pair);
           k_decode_planes<true><<<2 * ctx->num_sms, kPlaneWarps * 32, 0, st>>>(p);
         }
         else
