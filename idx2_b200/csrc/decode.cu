@@ -723,8 +723,9 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   // registers hold one 4^3 block per lane, so 2D bricks, whose blocks are 4 x 4, keep
   // k_decode_level, as do several planes per key (other tables) and the coefficient mode.
   const bool by_lane = !r0.is2d && r0.bpc == 1 && !coeff_out;
-  const size_t smem = by_lane ? sizeof(brick_smem) : dec_smem_bytes(true, r0.f32);
-  cudaFuncSetAttribute(k_decode_bricks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem));
+  const size_t smem = by_lane ? sizeof(brick_smem<8>) : dec_smem_bytes(true, r0.f32);
+  cudaFuncSetAttribute(k_decode_bricks<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<8>));
+  cudaFuncSetAttribute(k_decode_bricks<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<16>));
   cudaFuncSetAttribute(k_decode_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
   cudaFuncSetAttribute(k_decode_level<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
   int occ3 = 0;
@@ -732,6 +733,29 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   {
     cudaGetLastError();
     occ3 = 0;
+  }
+  auto launch_bricks = [&](const dec_args& a, int grid, bool three) {
+    // A launch that leaves each brick an SM of its own takes 16 warps per brick (36 bricks: 45
+    // against 57 us); more bricks take 8, two bricks per SM (at 1024^3 the two measured alike).
+    if (by_lane && a.nbricks <= ctx->num_sms)
+      k_decode_bricks<16><<<grid, 512, sizeof(brick_smem<16>), st>>>(a);
+    else if (by_lane)
+      k_decode_bricks<8><<<grid, 256, sizeof(brick_smem<8>), st>>>(a);
+    else
+      (three ? k_decode_level<3> : k_decode_level<2>)<<<grid, kThreads, smem, st>>>(a);
+  };
+  // A grid whose every sample lies in a decoded brick is written whole; others (bricks absent
+  // from the dataset) start from zeros.
+  std::vector<char> covered(n, 0);
+  for (size_t i = 0; i < n && !coeff_out && !keep; ++i)
+  {
+    long long got = 0;
+    for (const decode_level& lv : rqs[i]->levels)
+      if (lv.is_output)
+        for (const decode_brick& b : lv.bricks)
+          got += (long long)b.dims[0] * b.dims[1] * b.dims[2];
+    const v3& od = rqs[i]->out_dims;
+    covered[i] = got == (long long)od.x * od.y * od.z && (size_t)got * out_elem == out_bytes[i];
   }
   // The levels run back to back without the host waiting in between: the host prepares a
   // level's tables while the previous level runs (stream order protects the device tables
@@ -741,7 +765,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   for (int attempt = 0; attempt < 4; ++attempt)
   {
     for (size_t i = 0; i < n; ++i)
-      if (out_bytes[i])
+      if (out_bytes[i] && !covered[i])
         cudaMemsetAsync(d_out[i], 0, out_bytes[i], st);
     if (coeff_out)
       cudaMemsetAsync(coeff_out, 0, (size_t)coeff_base[(size_t)L] * (size_t)NB * (r0.f32 ? 4 : 8), st);
@@ -995,7 +1019,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
           ag.nbricks = cuts[g + 1] - cuts[g];
           ag.unit_off = d_uoff + (size_t)cuts[g] * (size_t)r0.nsb;
           const int gg = ag.nbricks < grid ? ag.nbricks : grid;
-          (by_lane ? k_decode_bricks : three ? k_decode_level<3> : k_decode_level<2>)<<<gg, kThreads, smem, st>>>(ag);
+          launch_bricks(ag, gg, three);
           ++ctx->launches;
           const size_t z_next =
             g + 2 < cuts.size() ? (size_t)hb[(size_t)cuts[g + 1]].dst_from[2] : (size_t)r0.out_dims.z;
@@ -1015,7 +1039,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       }
       else
       {
-        (by_lane ? k_decode_bricks : three ? k_decode_level<3> : k_decode_level<2>)<<<grid, kThreads, smem, st>>>(a);
+        launch_bricks(a, grid, three);
         ctx->launches += 3;
       }
       cudaEventRecord(t1, st);

@@ -46,6 +46,7 @@ constexpr int kHighPlanes = 26;  // planes the high words alone hold exactly
 constexpr int kLowBase = 14;     // bit of weight 1 in the second part's words
 constexpr int kSplitPlanes = 44; // planes that the two parts hold together
 
+template <int W>
 struct brick_smem
 {
   union alignas(16)
@@ -54,14 +55,14 @@ struct brick_smem
     long long q[64];           // one block (more than kSplitPlanes planes)
     double plane[kFace];       // a z-plane between its y and x sweeps
     float rows[32 * 36];       // its rows cast to float, 144 bytes each
-  } w[kWarps];
+  } w[W];
   double face[3][kFace];       // samples at x = 32 ([z][y]), y = 32 ([z][x]), z = 32 ([y][x])
-  double scale[kWarps][32];    // dequantisation of the task's blocks, by lane
+  double scale[W][32];    // dequantisation of the task's blocks, by lane
   uint8_t block[8][128];       // block of (zb * 5 + yb) * 5 + xb in the subband's walk, 255: not coded
   decode_target rq;
   int sig;
 };
-static_assert(sizeof(brick_smem::w[0]) % 16 == 0, "every warp's rows start 16-byte aligned");
+static_assert(sizeof(brick_smem<1>::w[0]) % 16 == 0, "every warp's rows start 16-byte aligned");
 
 __device__ __forceinline__ int slot_xy(int x, int y)
 {
@@ -218,7 +219,8 @@ struct lane_block
   const unsigned long long* row;
 };
 
-__device__ __forceinline__ lane_block find_block(const dec_args& a, const brick_smem& sm, const decode_brick& br,
+template <int W>
+__device__ __forceinline__ lane_block find_block(const dec_args& a, const brick_smem<W>& sm, const decode_brick& br,
                                                  int bi, int s, int xb, int yb, int zb, bool there)
 {
   lane_block lb;
@@ -251,7 +253,8 @@ __device__ __forceinline__ double dequant_scale(int nd, int emax)
 
 // The faces: 2D blocks (tasks 0-5: faces x, y, z, by the parity of the second axis), then the
 // edges and the corner (task 6), a lane per block.
-__device__ __forceinline__ void rebuild_face(const dec_args& a, brick_smem& sm, const decode_brick& br, int bi,
+template <int W>
+__device__ __forceinline__ void rebuild_face(const dec_args& a, brick_smem<W>& sm, const decode_brick& br, int bi,
                                              int task, int lane, bool sig_level)
 {
   if (task < 6)
@@ -407,7 +410,8 @@ __device__ __forceinline__ void lift_column(double (&v)[33], const dec_args& a, 
 
 // One task of the rebuild: parities (hx, hy) and block row yb, the 4 tiles along x: 32 blocks
 // (a lane each: tile t, z block zb, z parity hz), then their 64 columns along z.
-__device__ __forceinline__ void rebuild_tiles(const dec_args& a, brick_smem& sm, const decode_brick& br, int bi,
+template <int W>
+__device__ __forceinline__ void rebuild_tiles(const dec_args& a, brick_smem<W>& sm, const decode_brick& br, int bi,
                                               int task, double* F, int warp, int lane, bool sig_level)
 {
   const int hx = task >> 3, hy = (task >> 2) & 1, yb = task & 3;
@@ -546,18 +550,19 @@ __device__ __forceinline__ void ilift33_lanes(double& e, double& o, int lane)
   o = __dadd_rn(o, __dmul_rn(lane < 15 ? __dadd_rn(e, r) : __dadd_rn(r, e), 0.5));
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_decode_bricks(const dec_args a)
+template <int W>
+__global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args a)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  brick_smem& sm = *reinterpret_cast<brick_smem*>(smem_raw);
+  brick_smem<W>& sm = *reinterpret_cast<brick_smem<W>*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* const F = a.slots + (size_t)blockIdx.x * (size_t)kSlotBrick;
   const bool sig_level = a.level + 1 == a.nlevels;
   // the level's block walk, by block position
-  for (int i = tid; i < 8 * 128; i += kThreads)
+  for (int i = tid; i < 8 * 128; i += 32 * W)
     (&sm.block[0][0])[i] = 255;
   __syncthreads();
-  for (int i = tid; i < 8 * kMaxBlocksPerSubband; i += kThreads)
+  for (int i = tid; i < 8 * kMaxBlocksPerSubband; i += 32 * W)
   {
     const int s = i / kMaxBlocksPerSubband, b = i % kMaxBlocksPerSubband;
     if (b >= a.nblocks[s])
@@ -573,7 +578,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_bricks(const dec_args a)
     {
       const uint32_t* src = reinterpret_cast<const uint32_t*>(a.reqs + br.req);
       uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.rq);
-      for (int i = tid; i < (int)(sizeof(decode_target) / 4); i += kThreads)
+      for (int i = tid; i < (int)(sizeof(decode_target) / 4); i += 32 * W)
         dst[i] = src[i];
     }
     if (tid == 0)
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_bricks(const dec_args a)
       rebuild_face(a, sm, br, bi, warp, lane, sig_level);
     __syncthreads();
     // 2: blocks and z sweep; the columns of the faces x = 32 and y = 32 (and their common one)
-    for (int t = warp; t < 19; t += kWarps)
+    for (int t = warp; t < 19; t += W)
     {
       if (t < 16)
       {
@@ -611,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_bricks(const dec_args a)
                       br.dst_strd[0] == 1 && br.dst_from[0] % 4 == 0 && rq.out_dims[0] % 4 == 0 &&
                       (reinterpret_cast<uintptr_t>(rq.out) & 15) == 0;
     const int nplanes = rq.is_output ? br.dims[2] : 33;
-    for (int p = warp; p < nplanes; p += kWarps)
+    for (int p = warp; p < nplanes; p += W)
     {
       const int z = rq.is_output ? br.src_from[2] + p * br.src_strd[2] : p;
       const double* const S = F + (size_t)z * kSlotPlane;

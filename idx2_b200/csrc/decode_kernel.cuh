@@ -585,24 +585,20 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, Pu
 // memory latency inside the chain. Every lane's stream therefore comes through a ring of 16
 // words in shared memory (word-major, so lanes never collide), refilled 16 bytes at a time a
 // step ahead: no load from global memory is waited for where it is used, and the bits at a
-// position are two shared loads and a funnel shift, without the branch at a word's end. A group
-// test and its run are one bit scan of a 32-bit window, with a bit planted where the run must
-// end.
+// position are two shared loads and a funnel shift, without the branch at a word's end. The
+// group tests within the next 12 bits come from a table, several coefficients at once; what it
+// does not hold (a longer run, the last coefficient) is one bit scan, with a bit planted where
+// the run must end.
 //
 // Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
-// 6.8 ms against 9.5 ms with 64-bit windows refilled from global memory where they ran out (153 K
-// against 221 K warp instructions per brick, 74% issue activity: what bounds it is instructions,
-// 9 of 32 lanes active, as every step waits for its longest plane); 64 units, where only the
-// chain counts, 145 against 350 us.
+// 6.5 ms against 9.5 ms with 64-bit windows refilled from global memory where they ran out (6.8
+// ms with the bit scan alone); 64 units, where only the chain counts, 124 against 350 us (145).
+// What bounds it is instructions: 74% issue activity with 9 of 32 lanes active, as every step
+// waits for its longest plane.
 // ---------------------------------------------------------------------------
 constexpr int kRingWords = 16;
 constexpr unsigned kRingMask = (kRingWords - 1) * 128;  // byte offset of a ring word, 32 lanes wide
 
-struct ring_smem
-{
-  uint32_t info[kPlaneWarps][2][kMaxBlocksPerSubband];  // top key value | planes << 16 | log2 values << 24
-  uint32_t ring[kPlaneWarps][kRingWords * 32];
-};
 
 // shifts that give 0 from 32 bits on
 __device__ __forceinline__ uint32_t shl_to0(uint32_t x, int n)
@@ -618,6 +614,45 @@ __device__ __forceinline__ uint32_t shr_to0(uint32_t x, int n)
   return r;
 }
 
+// The group tests that 12 bits of a stream hold from a test bit on: bit r is set when coefficient
+// n + r is found significant (its test bit and run, with the one that ends it, lie within the 12
+// bits), kTestsEnd when a test bit of 0 ends the plane. A coefficient at distance r takes r + 1
+// run bits and a test bit for each one found: the bits read follow from the set bits alone.
+constexpr int kTestBits = 12;
+constexpr uint32_t kTestsEnd = 1u << 15;
+struct alignas(16) test_table
+{
+  uint16_t v[1 << kTestBits];
+};
+constexpr test_table make_test_table()
+{
+  test_table t{};
+  for (int x = 0; x < (1 << kTestBits); ++x)
+  {
+    uint32_t e = 0;
+    int at = 0, r = 0;
+    while (at < kTestBits)
+    {
+      if (!((x >> at) & 1))
+      {
+        e |= kTestsEnd;
+        break;
+      }
+      int z = 0;
+      while (at + 1 + z < kTestBits && !((x >> (at + 1 + z)) & 1))
+        ++z;
+      if (at + 1 + z >= kTestBits)
+        break;
+      e |= 1u << (r + z);
+      r += z + 1;
+      at += z + 2;
+    }
+    t.v[x] = (uint16_t)e;
+  }
+  return t;
+}
+__device__ const test_table kTestTable = make_test_table();
+
 // 32 bits of the lane's stream from bit position p of its ring
 __device__ __forceinline__ uint32_t ring_peek(const uint32_t* ring, uint32_t p)
 {
@@ -629,8 +664,8 @@ __device__ __forceinline__ uint32_t ring_peek(const uint32_t* ring, uint32_t p)
 
 // One bit plane (Core/Zfp.h:990 Decode<u64>) from position p: at most 128 bits. The plane's bits
 // in (xlo, xhi); n (significant coefficients) and p advance.
-__device__ __forceinline__ void ring_plane(const uint32_t* ring, uint32_t& p, int& n, int nvals, uint32_t& xlo,
-                                           uint32_t& xhi)
+__device__ __forceinline__ void ring_plane(const uint32_t* ring, const uint16_t* tests, uint32_t& p, int& n, int nvals,
+                                           uint32_t& xlo, uint32_t& xhi)
 {
   xlo = 0;
   xhi = 0;
@@ -644,57 +679,60 @@ __device__ __forceinline__ void ring_plane(const uint32_t* ring, uint32_t& p, in
   if (n >= nvals)
     return;
   const int last = nvals - 1;
-  uint32_t g = ring_peek(ring, p);  // the window: `rem` of its bits are left, from position p + 32 - rem
-  int rem = 32;
   do
   {
-    if (rem < 16)
-    {
-      p += (uint32_t)(32 - rem);
-      g = ring_peek(ring, p);
-      rem = 32;
-    }
-    if (!(g & 1u))
-    {
-      --rem;
-      break;
-    }
-    // the run of zeros up to the next significant coefficient; it ends by itself at the last one
+    const uint32_t g = ring_peek(ring, p);
+    const uint32_t e = tests[g & ((1u << kTestBits) - 1u)];
+    // coefficients before the last one (the last one's run has no end bit)
     const int lim = last - n;
-    const uint32_t h = (g >> 1) | shl_to0(1u, lim);
-    int z = __ffs((int)h) - 1;
-    if ((unsigned)z >= (unsigned)(rem - 1))
+    const uint32_t found = e & (kTestsEnd - 1u), take = found & ~shl_to0(~0u, lim);
+    if (take == 0 && e != kTestsEnd)
     {
-      // it leaves the window
-      p += (uint32_t)(33 - rem);
-      const uint32_t lo = ring_peek(ring, p), hi = ring_peek(ring, p + 32);
-      z = lo ? __ffs((int)lo) - 1 : (hi ? 31 + __ffs((int)hi) : 64);
-      z = z < lim ? z : lim;
-      p += (uint32_t)(z + 1);
-      g = ring_peek(ring, p);
-      rem = 32;
+      // one test and its run, which the table does not hold (or the last coefficient's): up to
+      // the next significant coefficient, or the last one
+      const uint32_t h = (g >> 1) | shl_to0(1u, lim);
+      int z = __ffs((int)h) - 1;
+      if (h == 0)
+      {
+        const uint32_t lo = ring_peek(ring, p + 32), hi = ring_peek(ring, p + 64);
+        z = lo ? 30 + __ffs((int)lo) : (hi ? 62 + __ffs((int)hi) : 64);
+        z = z < lim ? z : lim;
+      }
+      n += z;
+      p += (uint32_t)(z + 2);
+      xlo |= shl_to0(1u, n);
+      xhi |= shl_to0(1u, n - 32);
+      ++n;
+      continue;
     }
-    else
+    xlo |= shl_to0(take, n);
+    xhi |= n < 32 ? __funnelshift_lc(take, 0u, n) : shl_to0(take, n - 32);
+    const int a = 32 - __clz((int)take);
+    n += a;
+    p += (uint32_t)(a + __popc(take));
+    if (e >= kTestsEnd && take == found)
     {
-      g = shr_to0(g, z + 2);
-      rem -= z + 2;
+      ++p;
+      return;
     }
-    n += z;
-    xlo |= shl_to0(1u, n);
-    xhi |= shl_to0(1u, n - 32);
-    ++n;
   } while (n < nvals);
-  p += (uint32_t)(32 - rem);
   if (n == nvals)
     --p;  // the last run has no end bit
 }
+
+struct ring_smem
+{
+  uint32_t info[kPlaneWarps][2][kMaxBlocksPerSubband];  // top key value | planes << 16 | log2 values << 24
+  uint32_t ring[kPlaneWarps][kRingWords * 32];
+  alignas(16) uint16_t tests[1 << kTestBits];
+};
 
 // The wavefront of up to 32 channels (lane c: channel c), or of two units of up to 16 (U and the
 // block table are then the lane's unit's, c the lane within its half): channel 0 is a unit's top
 // key, where every block starts without significant coefficients, so what the shuffle brings
 // across from the other unit is not used.
 __device__ __forceinline__ void plane_wavefront_ring(const dec1_args& a, const plane_unit& U, const uint32_t* info,
-                                                     uint32_t* ring, int c, int steps)
+                                                     const uint16_t* tests, uint32_t* ring, int c, int steps)
 {
   const int nkeys = U.nkeys, nb = U.nb, key = U.kmax - c;
   bool has = false;
@@ -765,7 +803,7 @@ __device__ __forceinline__ void plane_wavefront_ring(const dec1_args& a, const p
           st = n | 256;
         else
         {
-          ring_plane(ring, p, n, 1 << (w >> 24), xlo, xhi);
+          ring_plane(ring, tests, p, n, 1 << (w >> 24), xlo, xhi);
           st = n;
         }
         row[kk] = ((unsigned long long)xhi << 32) | xlo;
@@ -782,6 +820,9 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 4) k_decode_planes_ring(cons
   __shared__ ring_smem sm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* const ring = sm.ring[warp] + lane;
+  for (int i = threadIdx.x; i < (int)(sizeof(test_table) / 16); i += kPlaneWarps * 32)
+    reinterpret_cast<uint4*>(sm.tests)[i] = reinterpret_cast<const uint4*>(kTestTable.v)[i];
+  __syncthreads();
   auto prep = [&](int unit, int which) {
     uint32_t* info = sm.info[warp][which];
     return prep_unit<false, false>(
@@ -799,7 +840,7 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 4) k_decode_planes_ring(cons
     const plane_unit U = prep(unit, 0);
     __syncwarp();
     if (U.run)
-      plane_wavefront_ring(a, U, sm.info[warp][0], ring, lane, U.nb + U.nkeys - 1);
+      plane_wavefront_ring(a, U, sm.info[warp][0], sm.tests, ring, lane, U.nb + U.nkeys - 1);
     return;
   }
   const int unit = a.unit_first + 2 * (blockIdx.x * kPlaneWarps + warp);
@@ -825,7 +866,7 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 4) k_decode_planes_ring(cons
     U.stride = h ? B.stride : A.stride;
     U.fs = h ? B.fs : A.fs;
     U.T = h ? B.T : A.T;
-    plane_wavefront_ring(a, U, sm.info[warp][h], ring, lane & 15, sA > sB ? sA : sB);
+    plane_wavefront_ring(a, U, sm.info[warp][h], sm.tests, ring, lane & 15, sA > sB ? sA : sB);
     return;
   }
 #pragma unroll 1
@@ -833,7 +874,7 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 4) k_decode_planes_ring(cons
   {
     const plane_unit& U = k ? B : A;
     if (U.run)
-      plane_wavefront_ring(a, U, sm.info[warp][k], ring, lane, k ? sB : sA);
+      plane_wavefront_ring(a, U, sm.info[warp][k], sm.tests, ring, lane, k ? sB : sA);
     __syncwarp();
   }
 }
