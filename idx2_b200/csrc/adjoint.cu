@@ -25,17 +25,27 @@
 // writes every coded block, so in 2D, where such a block would keep the parent's values, D
 // and the decode agree only where every low-band block below the coarsest level is decoded.
 //
-// Kernels. A 3D brick is worked on by a cluster of kCS CTAs, CTA r holding planes
-// z in [8r, 8r + 8) of it in shared memory (the last CTA also plane 32): every zfp block spans
-// 8 planes along z (4 samples at stride 2), so each block lies inside one CTA. The inverse zfp
-// runs in place as 4-point lines along z, y and x over every block (a block of extent 1 along
-// an axis has no line there); the forward pass then writes the parent's values over the
-// uncoded blocks, the adjoint clears them before its transposed zfp. The one-level CDF5/3 runs
-// along y and x inside each CTA and along z over the cluster's distributed shared memory; that
-// Z pass writes the grid (finest level) or the kept brick straight from registers, and in the
-// adjoint reads the grid's gradient the same way. A 2D brick is one CTA: X pass inside, Y pass
-// as the column pass. The order of the three CDF passes differs from the decode's Z, Y, X:
-// they act on different axes and commute, the results differ by rounding only.
+// Kernels. A 3D brick lies in shared memory whole (float, one CTA) or over a cluster of two CTAs
+// (double: planes 0-15 and 16-32), rows 34 and planes 34 x 34 samples apart. The inverse zfp
+// takes a lane per 4^3 block, 64 samples in registers: a warp's 32 blocks are the 8 parities of
+// the 4 blocks of a row along x, whose samples at one place in the block lie in 32 different
+// banks (8 t + hx + 2 hy + 4 hz). Samples at x = 32, y = 32 and z = 32 (blocks of extent 1 on an
+// axis) go as 4-point lines, one axis after the other. The forward pass writes the parent's
+// values over the uncoded blocks, the adjoint hands theirs to the parent and clears them. The
+// one-level CDF5/3 runs along y, x (rows read two samples at a time, which an even row length
+// of 17 pairs leaves free of conflicts) and z; the Z pass writes the grid (finest level) or the
+// kept brick straight from registers, and in the adjoint reads the grid's gradient the same way;
+// the cluster's two halves meet in it only, through distributed shared memory. The next brick is
+// prefetched into L2 while this one is worked on. A 2D brick is one CTA: X pass inside, Y pass as
+// the column pass. The order of the three CDF passes differs from the decode's Z, Y, X: they act
+// on different axes and commute, the results differ by rounding only.
+//
+// What bounds it: per brick 29 K cycles forward, of which the shared-memory pipe is busy half
+// (some 10 accesses a sample) and the issue slots a third (38 K warp instructions), with the load
+// of a brick and the store of its grid not overlapped (one brick fills an SM). For 32 float fields
+// of 256^3 (gpu__time_duration, both levels) 1.86 ms forward and 2.18 ms adjoint; clusters of four
+// CTAs with every zfp pass and every sweep through shared memory took 3.09 and 2.69 ms, this
+// form over clusters of two CTAs, two clusters per SM pair, 2.09 and 2.26 ms.
 #include "codec_device.cuh"
 #include "device.h"
 #include "encoder.h"
@@ -44,8 +54,6 @@
 #include <cooperative_groups.h>
 
 #include <cstring>
-#include <set>
-#include <tuple>
 #include <vector>
 
 namespace cg = cooperative_groups;
@@ -56,22 +64,26 @@ namespace idx2g
 namespace
 {
 
-constexpr int kSynThreads = 320;
 constexpr int kPlane = 33 * 33;
-constexpr int kCS = 4;   // CTAs per 3D brick (a thread-block cluster)
-constexpr int kPPC = 8;  // planes per CTA; the last CTA of the cluster also holds plane 32
+constexpr int kRow = 34;            // samples between rows of a brick in shared memory
+constexpr int kLayer = 34 * kRow;   // and between its planes
+constexpr int kSynThreads2 = 320;   // 2D bricks
 
+// 3D: CTAs per brick, threads per CTA (the 1,089 lines of a sweep, or a half's 561, take two
+// rounds)
 template <typename T>
-constexpr int syn_ctas_per_sm()
+struct syn3
 {
-  return sizeof(T) == 4 ? 3 : 2;
-}
+  static constexpr int CS = sizeof(T) == 4 ? 1 : 2;
+  static constexpr int threads = sizeof(T) == 4 ? 576 : 288;
+  static constexpr size_t smem = (size_t)(sizeof(T) == 4 ? 33 : 17) * kLayer * sizeof(T);
+};
 
 struct syn_brick
 {
   int b3[3];
   int valid[3];   // samples of the grid in the brick (finest level)
-  int parent;     // index of the parent brick on the coarser level (all fields), -1 if none
+  int parent;     // index of the parent brick on the coarser level (all fields)
   int pos[3];     // position inside the parent (0/1 per axis)
   int field;
   long long coff; // offset of the brick in its field's coefficient tensor (elements)
@@ -82,7 +94,8 @@ struct syn_args
 {
   int nbricks, coarsest, finest, norm_mask;
   double inv_weight[8];
-  const syn_brick* bricks;
+  int nb[3], npb[3];     // bricks per axis of one field on this level and on the coarser one
+  long long cbase;       // first element of the level in a field's coefficient tensor
   long long cstride;     // elements of one field's coefficient tensor
   long long gstride;     // elements of one field's grid
   long long gdims[3];
@@ -97,63 +110,85 @@ struct syn_args
   T* bricks_out;
 };
 
+// Brick bi of the launch: the fields one after the other, row-major bricks (x fastest) in each.
+template <typename T>
+__device__ __forceinline__ syn_brick brick_at(const syn_args<T>& a, int bi, bool is2d)
+{
+  syn_brick b;
+  const int per = a.nb[0] * a.nb[1] * a.nb[2];
+  b.field = bi / per;
+  const int i = bi - b.field * per, r = i / a.nb[0];
+  b.b3[0] = i - r * a.nb[0];
+  b.b3[2] = r / a.nb[1];
+  b.b3[1] = r - b.b3[2] * a.nb[1];
+  for (int k = 0; k < 3; ++k)
+  {
+    const int side = is2d && k == 2 ? 1 : 32;
+    const long long left = a.gdims[k] - (long long)b.b3[k] * side;
+    b.valid[k] = (int)(left < side ? left : side);
+    b.pos[k] = is2d && k == 2 ? 0 : b.b3[k] & 1;
+  }
+  const int pz = is2d ? b.b3[2] : b.b3[2] >> 1;
+  b.parent = b.field * (a.npb[0] * a.npb[1] * a.npb[2]) + (pz * a.npb[1] + (b.b3[1] >> 1)) * a.npb[0] + (b.b3[0] >> 1);
+  b.coff = a.cbase + (long long)i * (is2d ? kPlane : 33 * kPlane);
+  return b;
+}
+
+// a * k + b for a power of two k: the product is exact, so this is the sum's one rounding
+__device__ __forceinline__ float axpb(float a, float k, float b) { return __fmaf_rn(a, k, b); }
+__device__ __forceinline__ double axpb(double a, double k, double b) { return __fma_rn(a, k, b); }
+
 // Real inverse zfp lifting of one 4-point line (Core/Zfp.h:181 ILift, halvings exact).
 template <typename T>
-__device__ __forceinline__ void rilift4(T* q, int s)
+__device__ __forceinline__ void rilift4(T& x, T& y, T& z, T& w)
 {
-  T x = q[0], y = q[s], z = q[2 * s], w = q[3 * s];
-  y += w * T(0.5);
-  w -= y * T(0.5);
+  y = axpb(w, T(0.5), y);
+  w = axpb(y, T(-0.5), w);
   y += w;
-  w *= T(2);
-  w -= y;
+  w = axpb(w, T(2), -y);
   z += x;
-  x *= T(2);
-  x -= z;
+  x = axpb(x, T(2), -z);
   y += z;
-  z *= T(2);
-  z -= y;
+  z = axpb(z, T(2), -y);
   w += x;
-  x *= T(2);
-  x -= w;
-  q[0] = x;
-  q[s] = y;
-  q[2 * s] = z;
-  q[3 * s] = w;
+  x = axpb(x, T(2), -w);
 }
 
 // Its transpose: the elementary steps of rilift4 transposed, in reverse order.
 template <typename T>
-__device__ __forceinline__ void rilift4_adj(T* q, int s)
+__device__ __forceinline__ void rilift4_adj(T& x, T& y, T& z, T& w)
+{
+  w -= x;
+  x = axpb(x, T(2), w);
+  y -= z;
+  z = axpb(z, T(2), y);
+  z -= x;
+  x = axpb(x, T(2), z);
+  y -= w;
+  w = axpb(w, T(2), y);
+  y = axpb(w, T(-0.5), y);
+  w = axpb(y, T(0.5), w);
+}
+
+template <typename T, bool ADJ>
+__device__ __forceinline__ void lift4(T& x, T& y, T& z, T& w)
+{
+  if constexpr (ADJ)
+    rilift4_adj(x, y, z, w);
+  else
+    rilift4(x, y, z, w);
+}
+
+// the same on samples s apart in shared memory
+template <typename T, bool ADJ>
+__device__ __forceinline__ void lift4_at(T* q, int s)
 {
   T x = q[0], y = q[s], z = q[2 * s], w = q[3 * s];
-  w -= x;
-  x *= T(2);
-  x += w;
-  y -= z;
-  z *= T(2);
-  z += y;
-  z -= x;
-  x *= T(2);
-  x += z;
-  y -= w;
-  w *= T(2);
-  w += y;
-  y -= w * T(0.5);
-  w += y * T(0.5);
+  lift4<T, ADJ>(x, y, z, w);
   q[0] = x;
   q[s] = y;
   q[2 * s] = z;
   q[3 * s] = w;
-}
-
-template <typename T, bool ADJ>
-__device__ __forceinline__ void lift4(T* q, int s)
-{
-  if constexpr (ADJ)
-    rilift4_adj(q, s);
-  else
-    rilift4(q, s);
 }
 
 // One-level inverse CDF5/3 of a 33-sample line (Core/Wavelet.h:250 ILiftCdf53, D = 33) and
@@ -162,38 +197,31 @@ template <typename T>
 __device__ __forceinline__ void rilift33(T (&v)[33])
 {
 #pragma unroll
-  for (int x = 1; x < 31; x += 2)
+  for (int x = 1; x < 33; x += 2)
   {
-    const T V = v[x] * T(0.25);
-    v[x - 1] -= V;
-    v[x + 1] -= V;
-  }
-  {
-    const T V = v[31] * T(0.25);
-    v[30] -= V;
-    v[32] -= V;
+    v[x - 1] = axpb(v[x], T(-0.25), v[x - 1]);
+    v[x + 1] = axpb(v[x], T(-0.25), v[x + 1]);
   }
 #pragma unroll
-  for (int x = 1; x < 31; x += 2)
-    v[x] += (v[x - 1] + v[x + 1]) * T(0.5);
-  v[31] += (v[32] + v[30]) * T(0.5);
+  for (int x = 1; x < 33; x += 2)
+    v[x] = axpb(v[x - 1] + v[x + 1], T(0.5), v[x]);
 }
 
 template <typename T>
 __device__ __forceinline__ void rilift33_adj(T (&g)[33])
 {
-  g[32] += g[31] * T(0.5);
-  g[30] += g[31] * T(0.5);
+  g[32] = axpb(g[31], T(0.5), g[32]);
+  g[30] = axpb(g[31], T(0.5), g[30]);
 #pragma unroll
   for (int x = 1; x < 31; x += 2)
   {
-    g[x - 1] += g[x] * T(0.5);
-    g[x + 1] += g[x] * T(0.5);
+    g[x - 1] = axpb(g[x], T(0.5), g[x - 1]);
+    g[x + 1] = axpb(g[x], T(0.5), g[x + 1]);
   }
-  g[31] -= (g[30] + g[32]) * T(0.25);
+  g[31] = axpb(g[30] + g[32], T(-0.25), g[31]);
 #pragma unroll
   for (int x = 1; x < 31; x += 2)
-    g[x] -= (g[x - 1] + g[x + 1]) * T(0.25);
+    g[x] = axpb(g[x - 1] + g[x + 1], T(-0.25), g[x]);
 }
 
 template <typename T, bool ADJ>
@@ -234,104 +262,180 @@ __device__ __forceinline__ void cluster_sync()
     __syncthreads();
 }
 
-// n contiguous values from global memory into shared memory (asynchronous copies, then a
-// barrier).
 template <typename T>
-__device__ __forceinline__ void load_planes(T* S, const T* src, int n, int tid)
+__device__ __forceinline__ void copy_async(T* dst, const T* src)
 {
-  const unsigned s0 = (unsigned)__cvta_generic_to_shared(S);
-  for (int i = tid; i < n; i += kSynThreads)
-  {
-    if constexpr (sizeof(T) == 4)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s0 + 4u * (unsigned)i), "l"(src + i)
-                   : "memory");
-    else
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s0 + 8u * (unsigned)i), "l"(src + i)
-                   : "memory");
-  }
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (sizeof(T) == 4)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void copy_wait()
+{
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
 }
 
-// Lines of the in-place inverse zfp (or its transpose) over the CTA's planes. Along z (3D):
-// the CTA's 8 planes are one block row per parity, planes hz + 2j. Along y and x: per plane
-// and parity h, blocks k = 0..3 at h + 8k + 2j; the fifth block of the 17-sample low half has
-// extent 1 and no line.
-template <typename T, bool ADJ>
-__device__ __forceinline__ void zfp_z(T* S, int tid)
+__device__ __forceinline__ void prefetch_l2(const void* p)
 {
-  for (int L = tid; L < 2 * kPlane; L += kSynThreads)
-  {
-    const int xy = L % kPlane, hz = L / kPlane;
-    lift4<T, ADJ>(S + hz * kPlane + xy, 2 * kPlane);
-  }
+  asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
 }
 
+// In-place inverse zfp (or its transpose) lines of a 2D brick, rows of 33: along y and x, per
+// parity h, blocks k = 0..3 at h + 8k + 2j; the fifth block of the 17-sample low half has extent 1
+// and no line.
 template <typename T, bool ADJ>
-__device__ __forceinline__ void zfp_y(T* S, int np, int tid)
+__device__ __forceinline__ void zfp_y2(T* S, int tid)
 {
-  const int n = 33 * np;
-  for (int L = tid; L < 8 * n; L += kSynThreads)
+  for (int L = tid; L < 8 * 33; L += kSynThreads2)
   {
-    const int xp = L % n, g = L / n;
-    const int x = xp % 33, p = xp / 33;
-    lift4<T, ADJ>(S + (p * 33 + (g & 1) + 8 * (g >> 1)) * 33 + x, 66);
+    const int x = L % 33, g = L / 33;
+    lift4_at<T, ADJ>(S + ((g & 1) + 8 * (g >> 1)) * 33 + x, 66);
   }
 }
 
 template <typename T, bool ADJ>
-__device__ __forceinline__ void zfp_x(T* S, int np, int tid)
+__device__ __forceinline__ void zfp_x2(T* S, int tid)
 {
-  const int n = 33 * np;
-  for (int L = tid; L < 8 * n; L += kSynThreads)
+  for (int L = tid; L < 8 * 33; L += kSynThreads2)
   {
-    const int row = L % n, g = L / n;
-    lift4<T, ADJ>(S + row * 33 + (g & 1) + 8 * (g >> 1), 2);
+    const int row = L % 33, g = L / 33;
+    lift4_at<T, ADJ>(S + row * 33 + (g & 1) + 8 * (g >> 1), 2);
   }
 }
 
-// CDF5/3 lines along y (per x and plane) and along x (per row) inside the CTA; DN applies the
-// de-normalisation before the lift (forward) or after the transposed lift (adjoint).
-template <typename T, bool IS2D, bool ADJ, bool DN>
-__device__ __forceinline__ void cdf_y(const T* sw, T* S, int np, int z0, int tid)
+// CDF5/3 lines along x of a 2D brick; the de-normalisation comes before the lift (forward) or
+// after the transposed lift (adjoint).
+template <typename T, bool ADJ>
+__device__ __forceinline__ void cdf_x2(const T* sw, T* S, int tid)
 {
-  for (int L = tid; L < 33 * np; L += kSynThreads)
+  for (int y = tid; y < 33; y += kSynThreads2)
   {
-    const int x = L % 33, p = L / 33, z = z0 + p;
-    T* col = S + p * kPlane + x;
-    T v[33];
-#pragma unroll
-    for (int y = 0; y < 33; ++y)
-      v[y] = (DN && !ADJ) ? col[y * 33] * sw[parity_index<IS2D>(x, y, z)] : col[y * 33];
-    lift33<T, ADJ>(v);
-#pragma unroll
-    for (int y = 0; y < 33; ++y)
-      col[y * 33] = (DN && ADJ) ? v[y] * sw[parity_index<IS2D>(x, y, z)] : v[y];
-  }
-}
-
-template <typename T, bool IS2D, bool ADJ, bool DN>
-__device__ __forceinline__ void cdf_x(const T* sw, T* S, int np, int z0, int tid)
-{
-  for (int L = tid; L < 33 * np; L += kSynThreads)
-  {
-    const int y = L % 33, z = z0 + L / 33;
-    T* row = S + L * 33;
+    T* row = S + y * 33;
     T v[33];
 #pragma unroll
     for (int x = 0; x < 33; ++x)
-      v[x] = (DN && !ADJ) ? row[x] * sw[parity_index<IS2D>(x, y, z)] : row[x];
+      v[x] = !ADJ ? row[x] * sw[parity_index<true>(x, y, 0)] : row[x];
     lift33<T, ADJ>(v);
 #pragma unroll
     for (int x = 0; x < 33; ++x)
-      row[x] = (DN && ADJ) ? v[x] * sw[parity_index<IS2D>(x, y, z)] : v[x];
+      row[x] = ADJ ? v[x] * sw[parity_index<true>(x, y, 0)] : v[x];
   }
 }
 
-// The cluster CTA holding plane z of the brick.
-__device__ __forceinline__ int plane_rank(int z)
+// The inverse zfp (or its transpose) of the 4^3 blocks of block row (yb, zb), a lane per block.
+// `low`: the blocks of the first subband are coded too.
+template <typename T, bool ADJ>
+__device__ __forceinline__ void zfp_blocks(T* S, int yb, int zb, bool low, int lane)
 {
-  return z < kPPC * (kCS - 1) ? z / kPPC : kCS - 1;
+  const int t = lane & 3, hx = (lane >> 2) & 1, hy = (lane >> 3) & 1, hz = lane >> 4;
+  T* b = S + (8 * zb + hz) * kLayer + (8 * yb + hy) * kRow + 8 * t + hx;
+  T q[64];
+#pragma unroll
+  for (int j = 0; j < 64; ++j)
+    q[j] = b[(j >> 4) * 2 * kLayer + ((j >> 2) & 3) * 2 * kRow + (j & 3) * 2];
+#pragma unroll
+  for (int pass = 0; pass < 3; ++pass)
+  {
+    const int s = (ADJ ? pass : 2 - pass) == 0 ? 1 : ((ADJ ? pass : 2 - pass) == 1 ? 4 : 16);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+    {
+      const int o = s == 1 ? 4 * i : (s == 4 ? (i & 3) + 16 * (i >> 2) : i);
+      lift4<T, ADJ>(q[o], q[o + s], q[o + 2 * s], q[o + 3 * s]);
+    }
+  }
+  if (!low && hx + hy + hz == 0)
+    return;
+#pragma unroll
+  for (int j = 0; j < 64; ++j)
+    b[(j >> 4) * 2 * kLayer + ((j >> 2) & 3) * 2 * kRow + (j & 3) * 2] = q[j];
+}
+
+// Lines of the blocks of extent 1 on an axis, the CTA's `np` planes (8 nzb of them in whole
+// blocks along z; `top`: the last one is plane 32).
+template <typename T, bool ADJ>
+__device__ __forceinline__ void face_z(T* S, int nzb, int tid, int nt)
+{
+  for (int L = tid; L < 65 * 2 * nzb; L += nt)
+  {
+    const int c = L % 65, g = L / 65;
+    const int x = c < 33 ? 32 : c - 33, y = c < 33 ? c : 32;
+    lift4_at<T, ADJ>(S + (8 * (g >> 1) + (g & 1)) * kLayer + y * kRow + x, 2 * kLayer);
+  }
+}
+
+template <typename T, bool ADJ>
+__device__ __forceinline__ void face_y(T* S, int np, bool top, int tid, int nt)
+{
+  const int n = np + (top ? 32 : 0);  // x = 32 on every plane, then plane 32
+  for (int L = tid; L < 8 * n; L += nt)
+  {
+    const int c = L % n, g = L / n;
+    const int x = c < np ? 32 : c - np, p = c < np ? c : np - 1;
+    lift4_at<T, ADJ>(S + p * kLayer + (8 * (g >> 1) + (g & 1)) * kRow + x, 2 * kRow);
+  }
+}
+
+template <typename T, bool ADJ>
+__device__ __forceinline__ void face_x(T* S, int np, bool top, int tid, int nt)
+{
+  const int n = np + (top ? 32 : 0);  // y = 32 on every plane, then plane 32
+  for (int L = tid; L < 8 * n; L += nt)
+  {
+    const int c = L % n, g = L / n;
+    const int y = c < np ? 32 : c - np, p = c < np ? c : np - 1;
+    lift4_at<T, ADJ>(S + p * kLayer + y * kRow + 8 * (g >> 1) + (g & 1), 2);
+  }
+}
+
+// CDF5/3 lines along y, with the de-normalisation before the lift (forward) or after the
+// transposed lift (adjoint).
+template <typename T, bool ADJ>
+__device__ __forceinline__ void cdf_y(const T* sw, T* S, int np, int z0, int tid, int nt)
+{
+  for (int L = tid; L < 33 * np; L += nt)
+  {
+    const int x = L % 33, p = L / 33;
+    const T w0 = sw[parity_index<false>(x, 0, z0 + p)], w1 = sw[parity_index<false>(x, 1, z0 + p)];
+    T* col = S + p * kLayer + x;
+    T v[33];
+#pragma unroll
+    for (int y = 0; y < 33; ++y)
+      v[y] = !ADJ ? col[y * kRow] * ((y & 1) ? w1 : w0) : col[y * kRow];
+    lift33<T, ADJ>(v);
+#pragma unroll
+    for (int y = 0; y < 33; ++y)
+      col[y * kRow] = ADJ ? v[y] * ((y & 1) ? w1 : w0) : v[y];
+  }
+}
+
+// CDF5/3 lines along x, two samples an access (the 34th is padding).
+template <typename T, bool ADJ>
+__device__ __forceinline__ void cdf_x(T* S, int np, int tid, int nt)
+{
+  struct alignas(2 * sizeof(T)) pair_t
+  {
+    T a, b;
+  };
+  for (int L = tid; L < 33 * np; L += nt)
+  {
+    pair_t* row = reinterpret_cast<pair_t*>(S + (L / 33) * kLayer + (L % 33) * kRow);
+    T v[33];
+#pragma unroll
+    for (int x = 0; x < 17; ++x)
+    {
+      const pair_t r = row[x];
+      v[2 * x] = r.a;
+      if (x < 16)
+        v[2 * x + 1] = r.b;
+    }
+    lift33<T, ADJ>(v);
+#pragma unroll
+    for (int x = 0; x < 17; ++x)
+      row[x] = pair_t{ v[2 * x], x < 16 ? v[2 * x + 1] : T(0) };
+  }
 }
 
 // Offset of the brick's first sample in a batch of grids.
@@ -344,102 +448,266 @@ __device__ __forceinline__ size_t grid_offset(const syn_args<T>& a, const syn_br
          (size_t)br.b3[0] * 32;
 }
 
-template <typename T, bool IS2D>
-__global__ void __launch_bounds__(kSynThreads, syn_ctas_per_sm<T>()) k_synth(const syn_args<T> a)
+// Shared-memory address of sample (z, c) of the brick, c the offset in a plane, in the CTA of the
+// cluster that holds plane z.
+template <typename T>
+__device__ __forceinline__ unsigned sample_addr(const unsigned* base, int z, int c)
+{
+  const int r = z < 16 ? 0 : 1;
+  return base[r] + (unsigned)(((z - 16 * r) * kLayer + c) * (int)sizeof(T));
+}
+
+template <typename T, bool ADJ>
+__global__ void __launch_bounds__(syn3<T>::threads, 1) k_synth3(const syn_args<T> a)
 {
   extern __shared__ __align__(16) unsigned char syn_smem[];
   __shared__ T sw[8];
+  __shared__ syn_brick sb[2];  // this brick and the next (made by one thread: some divisions)
   T* S = reinterpret_cast<T*>(syn_smem);
-  constexpr int CS = IS2D ? 1 : kCS;
-  const int tid = threadIdx.x;
+  constexpr int CS = syn3<T>::CS, NT = syn3<T>::threads, NW = NT / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   stage_weights(a, sw, tid);
   int rank = 0;
-  unsigned base[CS];  // the cluster's brick planes, as shared::cluster addresses
+  unsigned base[2] = { 0, 0 };  // the cluster's brick halves, as shared::cluster addresses
   if constexpr (CS > 1)
   {
     rank = (int)cg::this_cluster().block_rank();
-#pragma unroll
-    for (int r = 0; r < CS; ++r)
-      base[r] = dev::cluster_addr(S, r);
+    base[0] = dev::cluster_addr(S, 0);
+    base[1] = dev::cluster_addr(S, 1);
     cluster_sync<CS>();  // every CTA of the cluster has started before any remote access
   }
-  const int z0 = IS2D ? 0 : rank * kPPC;
-  const int np = IS2D ? 1 : (rank == CS - 1 ? 33 - z0 : kPPC);
-  const size_t NB = IS2D ? kPlane : 33 * kPlane;
+  const int z0 = rank * 16;
+  const int np = CS == 1 ? 33 : 16 + rank;
+  const int nzb = CS == 1 ? 4 : 2;
+  const bool top = rank == CS - 1;
   const int nclusters = gridDim.x / CS;
-  for (int bi = blockIdx.x / CS; bi < a.nbricks; bi += nclusters)
+  const size_t zs = (size_t)a.gdims[1] * (size_t)a.gdims[0];
+  if (tid == 0)
+    sb[0] = brick_at(a, (int)blockIdx.x / CS, false);
+  __syncthreads();
+  int cur = 0;
+  for (int bi = blockIdx.x / CS; bi < a.nbricks; bi += nclusters, cur ^= 1)
   {
-    const syn_brick& br = a.bricks[bi];
-    load_planes(S, a.in + (size_t)br.field * (size_t)a.cstride + (size_t)br.coff + (size_t)z0 * kPlane,
-                np * kPlane, tid);
-    // inverse zfp of every block, in place: z, y, x
-    if constexpr (!IS2D)
+    const syn_brick& br = sb[cur];
+    const int next = bi + nclusters;
+    if (tid == 0 && next < a.nbricks)
+      sb[cur ^ 1] = brick_at(a, next, false);  // read after the next barrier
+    const size_t cat = (size_t)br.field * (size_t)a.cstride + (size_t)br.coff + (size_t)z0 * kPlane;
+    if constexpr (!ADJ)
     {
-      zfp_z<T, false>(S, tid);
+      // the coefficients, a warp per row, the 33rd samples after them
+      const T* src = a.in + cat;
+      for (int y = warp; y < 33; y += NW)
+      {
+        const T* g = src + y * 33 + lane;
+        T* d = S + y * kRow + lane;
+#pragma unroll
+        for (int p = 0; p < (CS == 1 ? 33 : 16); ++p)
+          copy_async(d + p * kLayer, g + p * kPlane);
+        if (CS > 1 && top)
+          copy_async(d + 16 * kLayer, g + 16 * kPlane);
+      }
+      for (int r = tid; r < 33 * np; r += NT)
+        copy_async(S + (r / 33) * kLayer + (r % 33) * kRow + 32, src + r * 33 + 32);
+      copy_wait();
       __syncthreads();
-    }
-    zfp_y<T, false>(S, np, tid);
-    __syncthreads();
-    zfp_x<T, false>(S, np, tid);
-    __syncthreads();
-    if constexpr (!IS2D)
-    {
-      // the parent's values over the uncoded full low-band blocks (even samples below 32 of
-      // this CTA's planes)
+      // inverse zfp: z, y, x
+      if (warp < 4 * nzb)
+        zfp_blocks<T, false>(S, warp & 3, warp >> 2, a.coarsest, lane);
+      face_z<T, false>(S, nzb, tid, NT);
       if (!a.coarsest)
       {
-        const T* P = a.parents + (size_t)br.parent * NB;
-        for (int i = tid; i < 4 * 256; i += kSynThreads)
+        // the parent's values over the uncoded full low-band blocks (even samples below 32)
+        const T* P = a.parents + (size_t)br.parent * (33 * kPlane);
+        for (int i = tid; i < 4 * nzb * 256; i += NT)
         {
           const int x = i & 15, y = (i >> 4) & 15, k = i >> 8;
-          const int zz = (z0 >> 1) + k;
-          S[((2 * k) * 33 + 2 * y) * 33 + 2 * x] =
-            P[((br.pos[2] * 16 + zz) * 33 + (br.pos[1] * 16 + y)) * 33 + (br.pos[0] * 16 + x)];
+          S[2 * k * kLayer + 2 * y * kRow + 2 * x] =
+            P[((br.pos[2] * 16 + (z0 >> 1) + k) * 33 + (br.pos[1] * 16 + y)) * 33 + (br.pos[0] * 16 + x)];
         }
-        __syncthreads();
       }
-      cdf_y<T, false, false, true>(sw, S, np, z0, tid);
       __syncthreads();
-      cdf_x<T, false, false, false>(sw, S, np, z0, tid);
-      cluster_sync<CS>();
-      // Z pass over the cluster: this CTA's share of the 33 x 33 columns
-      constexpr int cpc = (kPlane + CS - 1) / CS;
-      for (int cl = tid; cl < cpc; cl += kSynThreads)
+      if (next < a.nbricks)
       {
-        const int c = rank * cpc + cl;
-        if (c >= kPlane)
-          break;
-        const int x = c % 33, y = c / 33;
+        const syn_brick& nx = sb[cur ^ 1];
+        const char* q = (const char*)(a.in + (size_t)nx.field * (size_t)a.cstride + (size_t)nx.coff +
+                                      (size_t)z0 * kPlane);
+        for (int k = tid * 128; k < np * kPlane * (int)sizeof(T); k += NT * 128)
+          prefetch_l2(q + k);
+      }
+      face_y<T, false>(S, np, top, tid, NT);
+      __syncthreads();
+      face_x<T, false>(S, np, top, tid, NT);
+      __syncthreads();
+      cdf_y<T, false>(sw, S, np, z0, tid, NT);
+      __syncthreads();
+      cdf_x<T, false>(S, np, tid, NT);
+      cluster_sync<CS>();
+      // Z pass over the brick: this CTA's share of the columns (the grid has those below 32)
+      const int side = a.finest ? 32 : 33;
+      for (int c = rank * NT + tid; c < side * side; c += CS * NT)
+      {
+        const int x = c % side, y = c / side, o = y * kRow + x;
         T v[33];
 #pragma unroll
         for (int z = 0; z < 33; ++z)
-          v[z] = dev::ld_cluster<T>(base[plane_rank(z)] + (unsigned)(((z - plane_rank(z) * kPPC) * kPlane + c) * sizeof(T)));
+        {
+          if constexpr (CS == 1)
+            v[z] = S[z * kLayer + o];
+          else
+            v[z] = dev::ld_cluster<T>(sample_addr<T>(base, z, o));
+        }
         rilift33(v);
         if (a.finest)
         {
           if (x < br.valid[0] && y < br.valid[1])
           {
             T* g = a.out + grid_offset(a, br, false) + (size_t)y * (size_t)a.gdims[0] + x;
-            const size_t zs = (size_t)a.gdims[1] * (size_t)a.gdims[0];
+            if (br.valid[2] == 32)
+            {
 #pragma unroll
-            for (int z = 0; z < 32; ++z)
-              if (z < br.valid[2])
-                g[(size_t)z * zs] = v[z];
+              for (int z = 0; z < 32; ++z, g += zs)
+                *g = v[z];
+            }
+            else
+            {
+#pragma unroll
+              for (int z = 0; z < 32; ++z, g += zs)
+                if (z < br.valid[2])
+                  *g = v[z];
+            }
           }
         }
         else
         {
-          T* o = a.bricks_out + (size_t)bi * NB + c;
+          T* out = a.bricks_out + (size_t)bi * (33 * kPlane) + c;
 #pragma unroll
           for (int z = 0; z < 33; ++z)
-            o[z * kPlane] = v[z];
+            out[z * kPlane] = v[z];
         }
       }
       cluster_sync<CS>();
     }
     else
     {
-      cdf_x<T, true, false, true>(sw, S, 1, 0, tid);
+      // transposed Z pass: this CTA's columns of the incoming gradient, into the cluster. The
+      // grid has those below 32; the faces x = 32 and y = 32 start from zeros there.
+      const int side = a.finest ? 32 : 33;
+      if (a.finest)
+        for (int i = tid; i < 65 * np; i += NT)
+        {
+          const int c = i % 65, p = i / 65;
+          S[p * kLayer + (c < 33 ? c * kRow + 32 : 32 * kRow + c - 33)] = T(0);
+        }
+      for (int c = rank * NT + tid; c < side * side; c += CS * NT)
+      {
+        const int x = c % side, y = c / side, o = y * kRow + x;
+        T v[33];
+        if (a.finest)
+        {
+          const int nz = x < br.valid[0] && y < br.valid[1] ? br.valid[2] : 0;  // valid[2] <= 32
+          const T* g = a.in + grid_offset(a, br, false) + (size_t)y * (size_t)a.gdims[0] + x;
+          v[32] = T(0);
+#pragma unroll
+          for (int z = 0; z < 32; ++z, g += zs)
+            v[z] = z < nz ? *g : T(0);
+        }
+        else
+        {
+          const T* gi = a.in + (size_t)bi * (33 * kPlane) + c;
+#pragma unroll
+          for (int z = 0; z < 33; ++z)
+            v[z] = gi[z * kPlane];
+        }
+        rilift33_adj(v);
+#pragma unroll
+        for (int z = 0; z < 33; ++z)
+        {
+          if constexpr (CS == 1)
+            S[z * kLayer + o] = v[z];
+          else
+            dev::st_cluster<T>(sample_addr<T>(base, z, o), v[z]);
+        }
+      }
+      cluster_sync<CS>();
+      if (next < a.nbricks && a.finest)
+      {
+        const syn_brick& nx = sb[cur ^ 1];
+        for (int r = rank * NT + tid; r < nx.valid[1] * nx.valid[2]; r += CS * NT)
+        {
+          const T* g = a.in + grid_offset(a, nx, false) + (size_t)(r % nx.valid[1]) * (size_t)a.gdims[0] +
+                       (size_t)(r / nx.valid[1]) * zs;
+          prefetch_l2(g);
+          prefetch_l2(g + nx.valid[0] - 1);
+        }
+      }
+      cdf_x<T, true>(S, np, tid, NT);
+      __syncthreads();
+      cdf_y<T, true>(sw, S, np, z0, tid, NT);
+      __syncthreads();
+      // transposed zfp: x, y, z; the low band over the uncoded blocks goes to the parent (and
+      // nowhere else)
+      face_x<T, true>(S, np, top, tid, NT);
+      if (!a.coarsest)
+      {
+        T* P = a.pgrad + (size_t)br.parent * (33 * kPlane);
+        for (int i = tid; i < 4 * nzb * 256; i += NT)
+        {
+          const int x = i & 15, y = (i >> 4) & 15, k = i >> 8;
+          T* s = S + 2 * k * kLayer + 2 * y * kRow + 2 * x;
+          P[((br.pos[2] * 16 + (z0 >> 1) + k) * 33 + (br.pos[1] * 16 + y)) * 33 + (br.pos[0] * 16 + x)] = *s;
+          *s = T(0);
+        }
+      }
+      __syncthreads();
+      face_y<T, true>(S, np, top, tid, NT);
+      __syncthreads();
+      if (warp < 4 * nzb)
+        zfp_blocks<T, true>(S, warp & 3, warp >> 2, a.coarsest, lane);
+      face_z<T, true>(S, nzb, tid, NT);
+      __syncthreads();
+      T* dst = a.out + cat;
+      for (int y = warp; y < 33; y += NW)
+      {
+        T* g = dst + y * 33 + lane;
+        const T* d = S + y * kRow + lane;
+#pragma unroll
+        for (int p = 0; p < (CS == 1 ? 33 : 16); ++p)
+          g[p * kPlane] = d[p * kLayer];
+        if (CS > 1 && top)
+          g[16 * kPlane] = d[16 * kLayer];
+      }
+      for (int r = tid; r < 33 * np; r += NT)
+        dst[r * 33 + 32] = S[(r / 33) * kLayer + (r % 33) * kRow + 32];
+      // the next brick's transposed Z pass writes into every CTA of the cluster
+      cluster_sync<CS>();
+    }
+  }
+}
+
+// 2D bricks: a CTA each.
+template <typename T, bool ADJ>
+__global__ void __launch_bounds__(kSynThreads2, sizeof(T) == 4 ? 3 : 2) k_synth2(const syn_args<T> a)
+{
+  __shared__ T S[kPlane];
+  __shared__ T sw[8];
+  const int tid = threadIdx.x;
+  stage_weights(a, sw, tid);
+  for (int bi = blockIdx.x; bi < a.nbricks; bi += gridDim.x)
+  {
+    const syn_brick br = brick_at(a, bi, true);
+    const size_t cat = (size_t)br.field * (size_t)a.cstride + (size_t)br.coff;
+    if constexpr (!ADJ)
+    {
+      for (int i = tid; i < kPlane; i += kSynThreads2)
+        copy_async(S + i, a.in + cat + i);
+      copy_wait();
+      __syncthreads();
+      zfp_y2<T, false>(S, tid);
+      __syncthreads();
+      zfp_x2<T, false>(S, tid);
+      __syncthreads();
+      cdf_x2<T, false>(sw, S, tid);
       __syncthreads();
       // Y pass: one column per x
       if (tid < 33)
@@ -463,97 +731,13 @@ __global__ void __launch_bounds__(kSynThreads, syn_ctas_per_sm<T>()) k_synth(con
         }
         else
         {
-          T* o = a.bricks_out + (size_t)bi * NB + x;
+          T* o = a.bricks_out + (size_t)bi * kPlane + x;
 #pragma unroll
           for (int y = 0; y < 33; ++y)
             o[y * 33] = v[y];
         }
       }
       __syncthreads();
-    }
-  }
-}
-
-template <typename T, bool IS2D>
-__global__ void __launch_bounds__(kSynThreads, syn_ctas_per_sm<T>()) k_synth_adj(const syn_args<T> a)
-{
-  extern __shared__ __align__(16) unsigned char syn_smem[];
-  __shared__ T sw[8];
-  T* S = reinterpret_cast<T*>(syn_smem);
-  constexpr int CS = IS2D ? 1 : kCS;
-  const int tid = threadIdx.x;
-  stage_weights(a, sw, tid);
-  int rank = 0;
-  unsigned base[CS];  // the cluster's brick planes, as shared::cluster addresses
-  if constexpr (CS > 1)
-  {
-    rank = (int)cg::this_cluster().block_rank();
-#pragma unroll
-    for (int r = 0; r < CS; ++r)
-      base[r] = dev::cluster_addr(S, r);
-    cluster_sync<CS>();  // every CTA of the cluster has started before any remote access
-  }
-  const int z0 = IS2D ? 0 : rank * kPPC;
-  const int np = IS2D ? 1 : (rank == CS - 1 ? 33 - z0 : kPPC);
-  const size_t NB = IS2D ? kPlane : 33 * kPlane;
-  const int nclusters = gridDim.x / CS;
-  for (int bi = blockIdx.x / CS; bi < a.nbricks; bi += nclusters)
-  {
-    const syn_brick& br = a.bricks[bi];
-    if constexpr (!IS2D)
-    {
-      // transposed Z pass: this CTA's columns of the incoming gradient, into the cluster
-      constexpr int cpc = (kPlane + CS - 1) / CS;
-      for (int cl = tid; cl < cpc; cl += kSynThreads)
-      {
-        const int c = rank * cpc + cl;
-        if (c >= kPlane)
-          break;
-        const int x = c % 33, y = c / 33;
-        T v[33];
-        if (a.finest)
-        {
-          const int nz = x < br.valid[0] && y < br.valid[1] ? br.valid[2] : 0;  // valid[2] <= 32
-          const T* g = a.in + grid_offset(a, br, false) + (size_t)y * (size_t)a.gdims[0] + x;
-          const size_t zs = (size_t)a.gdims[1] * (size_t)a.gdims[0];
-#pragma unroll
-          for (int z = 0; z < 33; ++z)
-          {
-            v[z] = z < nz ? *g : T(0);
-            g += zs;
-          }
-        }
-        else
-        {
-          const T* gi = a.in + (size_t)bi * NB + c;
-#pragma unroll
-          for (int z = 0; z < 33; ++z)
-            v[z] = gi[z * kPlane];
-        }
-        rilift33_adj(v);
-#pragma unroll
-        for (int z = 0; z < 33; ++z)
-          dev::st_cluster<T>(base[plane_rank(z)] + (unsigned)(((z - plane_rank(z) * kPPC) * kPlane + c) * sizeof(T)), v[z]);
-      }
-      cluster_sync<CS>();
-      cdf_x<T, false, true, false>(sw, S, np, z0, tid);
-      __syncthreads();
-      cdf_y<T, false, true, true>(sw, S, np, z0, tid);
-      __syncthreads();
-      // the low band over the uncoded blocks goes to the parent (and nowhere else)
-      if (!a.coarsest)
-      {
-        T* P = a.pgrad + (size_t)br.parent * NB;
-        for (int i = tid; i < 4 * 256; i += kSynThreads)
-        {
-          const int x = i & 15, y = (i >> 4) & 15, k = i >> 8;
-          const int zz = (z0 >> 1) + k;
-          T* s = S + ((2 * k) * 33 + 2 * y) * 33 + 2 * x;
-          P[((br.pos[2] * 16 + zz) * 33 + (br.pos[1] * 16 + y)) * 33 + (br.pos[0] * 16 + x)] = *s;
-          *s = T(0);
-        }
-        __syncthreads();
-      }
     }
     else
     {
@@ -571,7 +755,7 @@ __global__ void __launch_bounds__(kSynThreads, syn_ctas_per_sm<T>()) k_synth_adj
         }
         else
         {
-          const T* gi = a.in + (size_t)bi * NB + x;
+          const T* gi = a.in + (size_t)bi * kPlane + x;
 #pragma unroll
           for (int y = 0; y < 33; ++y)
             v[y] = gi[y * 33];
@@ -582,33 +766,26 @@ __global__ void __launch_bounds__(kSynThreads, syn_ctas_per_sm<T>()) k_synth_adj
           S[y * 33 + x] = v[y];
       }
       __syncthreads();
-      cdf_x<T, true, true, true>(sw, S, 1, 0, tid);
+      cdf_x2<T, true>(sw, S, tid);
+      __syncthreads();
+      zfp_x2<T, true>(S, tid);
+      __syncthreads();
+      zfp_y2<T, true>(S, tid);
+      __syncthreads();
+      for (int i = tid; i < kPlane; i += kSynThreads2)
+        a.out[cat + i] = S[i];
       __syncthreads();
     }
-    // transposed zfp: x, y, z
-    zfp_x<T, true>(S, np, tid);
-    __syncthreads();
-    zfp_y<T, true>(S, np, tid);
-    __syncthreads();
-    if constexpr (!IS2D)
-    {
-      zfp_z<T, true>(S, tid);
-      __syncthreads();
-    }
-    T* Gc = a.out + (size_t)br.field * (size_t)a.cstride + (size_t)br.coff + (size_t)z0 * kPlane;
-    for (int i = tid; i < np * kPlane; i += kSynThreads)
-      Gc[i] = S[i];
-    // the next brick's transposed Z pass writes into every CTA of the cluster
-    cluster_sync<CS>();
   }
 }
 
 // Bricks and weights of every level of a format (levels finest first).
 struct syn_level
 {
-  std::vector<syn_brick> bricks;  // one field
-  double inv_weight[8] = {};
-  int norm_mask = 0;
+  int nb[3];        // bricks per axis
+  long long base;   // first element of the level in a field's coefficient tensor
+  double inv_weight[8];
+  int norm_mask;
 };
 
 // The kernels assume the block layout of an extended brick: subband s at the parities of its
@@ -629,24 +806,23 @@ bool uniform_blocks(const dataset_format& f, int level)
     const v3 want(17 - h[0], 17 - h[1], is2d ? 1 : 17 - h[2]);
     if (!(sb.g.dims == want))
       return false;
-    std::set<std::tuple<int, int, int, int, int, int>> expect, got;
     const int nk[3] = { h[0] ? 4 : 5, h[1] ? 4 : 5, is2d ? 1 : (h[2] ? 4 : 5) };
-    for (int kz = 0; kz < nk[2]; ++kz)
-      for (int ky = 0; ky < nk[1]; ++ky)
-        for (int kx = 0; kx < nk[0]; ++kx)
-        {
-          const int bx = kx < 4 ? 4 : 1, by = ky < 4 ? 4 : 1, bz = is2d ? 1 : (kz < 4 ? 4 : 1);
-          const bool full = bx == 4 && by == 4 && bz == 4;
-          if (s == 0 && level + 1 < f.nlevels && full)
-            continue;
-          expect.insert(std::make_tuple(kx, ky, kz, bx, by, bz));
-        }
+    const size_t uncoded = s == 0 && level + 1 < f.nlevels && !is2d ? 64 : 0;
+    bool seen[125] = {};
     std::vector<block_geom> g;
     subband_blocks(f, level, s, &g);
-    for (const block_geom& b : g)
-      got.insert(std::make_tuple((int)b.dx, (int)b.dy, (int)b.dz, (int)b.bx, (int)b.by, (int)b.bz));
-    if (got != expect || got.size() != g.size())
+    if (g.size() + uncoded != (size_t)(nk[0] * nk[1] * nk[2]))
       return false;
+    for (const block_geom& b : g)
+    {
+      if (b.dx >= nk[0] || b.dy >= nk[1] || b.dz >= nk[2])
+        return false;
+      const int bx = b.dx < 4 ? 4 : 1, by = b.dy < 4 ? 4 : 1, bz = is2d ? 1 : (b.dz < 4 ? 4 : 1);
+      bool& at = seen[(b.dz * 5 + b.dy) * 5 + b.dx];
+      if (at || b.bx != bx || b.by != by || b.bz != bz || (uncoded && bx == 4 && by == 4 && bz == 4))
+        return false;
+      at = true;
+    }
   }
   return true;
 }
@@ -654,7 +830,10 @@ bool uniform_blocks(const dataset_format& f, int level)
 long long build_levels(const dataset_format& f, std::vector<syn_level>* out)
 {
   const int L = f.nlevels;
-  const int NB = f.is2d() ? 33 * 33 : 33 * 33 * 33;
+  const bool is2d = f.is2d();
+  const int NB = is2d ? 33 * 33 : 33 * 33 * 33;
+  if (L > 1 && !(f.group_brick3 == v3(2, 2, is2d ? 1 : 2)))
+    return -1;
   out->assign((size_t)L, syn_level());
   long long base = 0;
   for (int l = 0; l < L; ++l)
@@ -663,35 +842,11 @@ long long build_levels(const dataset_format& f, std::vector<syn_level>* out)
       return -1;
     syn_level& sl = (*out)[(size_t)l];
     const v3 n3 = f.nbricks3[(size_t)l];
-    const v3 np3 = l + 1 < L ? f.nbricks3[(size_t)l + 1] : v3(1);
-    for (int bz = 0; bz < n3.z; ++bz)
-      for (int by = 0; by < n3.y; ++by)
-        for (int bx = 0; bx < n3.x; ++bx)
-        {
-          syn_brick b;
-          memset(&b, 0, sizeof b);
-          b.b3[0] = bx;
-          b.b3[1] = by;
-          b.b3[2] = bz;
-          const v3 b3(bx, by, bz);
-          const v3 v = vmin(f.brick_dims, f.dims - b3 * f.brick_dims);
-          b.valid[0] = v.x;
-          b.valid[1] = v.y;
-          b.valid[2] = v.z;
-          if (l + 1 < L)
-          {
-            const v3 p3 = b3 / f.group_brick3, pos = b3 % f.group_brick3;
-            b.parent = (p3.z * np3.y + p3.y) * np3.x + p3.x;
-            b.pos[0] = pos.x;
-            b.pos[1] = pos.y;
-            b.pos[2] = pos.z;
-          }
-          else
-            b.parent = -1;
-          b.coff = base;
-          base += NB;
-          sl.bricks.push_back(b);
-        }
+    sl.nb[0] = n3.x;
+    sl.nb[1] = n3.y;
+    sl.nb[2] = n3.z;
+    sl.base = base;
+    base += (long long)n3.x * n3.y * n3.z * NB;
     double w[8];
     level_weights(f, l, w, &sl.norm_mask);
     for (int s = 0; s < 8; ++s)
@@ -703,37 +858,46 @@ long long build_levels(const dataset_format& f, std::vector<syn_level>* out)
 template <typename T, bool IS2D>
 int launch_synth(device_ctx* ctx, const syn_args<T>& a, bool adjoint, cudaStream_t st)
 {
-  constexpr int CS = IS2D ? 1 : kCS;
-  const size_t smem = (size_t)(IS2D ? 1 : kPPC + 1) * kPlane * sizeof(T);
-  void (*kern)(const syn_args<T>) = adjoint ? k_synth_adj<T, IS2D> : k_synth<T, IS2D>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return CudaError;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof cfg);
-  cudaLaunchAttribute attr[1];
-  cfg.blockDim = dim3(kSynThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  int nclusters = ctx->num_sms * syn_ctas_per_sm<T>() / CS;
-  if (CS > 1)
-  {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CS;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(CS * nclusters);
-    int active = 0;
-    if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active > 0)
-      nclusters = active;
-  }
-  if (nclusters > a.nbricks)
-    nclusters = a.nbricks;
-  if (nclusters < 1)
+  if (a.nbricks < 1)
     return NoError;
-  cfg.gridDim = dim3(CS * nclusters);
-  return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? NoError : CudaError;
+  if constexpr (IS2D)
+  {
+    const int grid = a.nbricks < 3 * ctx->num_sms ? a.nbricks : 3 * ctx->num_sms;
+    (adjoint ? k_synth2<T, true> : k_synth2<T, false>)<<<grid, kSynThreads2, 0, st>>>(a);
+    return cudaGetLastError() == cudaSuccess ? NoError : CudaError;
+  }
+  else
+  {
+    constexpr int CS = syn3<T>::CS;
+    const size_t smem = syn3<T>::smem;
+    void (*kern)(const syn_args<T>) = adjoint ? k_synth3<T, true> : k_synth3<T, false>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return CudaError;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute attr[1];
+    cfg.blockDim = dim3(syn3<T>::threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    int nclusters = ctx->num_sms / CS;
+    if (CS > 1)
+    {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = CS;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      cfg.gridDim = dim3(CS * nclusters);
+      int active = 0;
+      if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active > 0)
+        nclusters = active;
+    }
+    if (nclusters > a.nbricks)
+      nclusters = a.nbricks;
+    cfg.gridDim = dim3(CS * nclusters);
+    return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? NoError : CudaError;
+  }
 }
 
 template <typename T>
@@ -748,43 +912,28 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
   const int NB = f.is2d() ? 33 * 33 : 33 * 33 * 33;
   cudaStream_t st = ctx->stream;
   const long long gcount = (long long)f.dims.x * f.dims.y * f.dims.z;
-  float total = 0;
   T* prev = nullptr;  // forward: kept bricks of the coarser level; adjoint: this level's gradient bricks
   for (int step = 0; step < L; ++step)
   {
     const int l = adjoint ? step : L - 1 - step;
     const syn_level& sl = lv[(size_t)l];
-    const int per = (int)sl.bricks.size();
-    const int nbr = per * nbatch;
-    std::vector<syn_brick> hb((size_t)nbr);
-    for (int fi = 0; fi < nbatch; ++fi)
-      for (int i = 0; i < per; ++i)
-      {
-        syn_brick b = sl.bricks[(size_t)i];
-        b.field = fi;
-        if (b.parent >= 0)
-          b.parent += fi * (int)lv[(size_t)l + 1].bricks.size();
-        hb[(size_t)fi * (size_t)per + (size_t)i] = b;
-      }
-    char nm[32];
-    snprintf(nm, sizeof nm, "syn.bricks%d", step & 1);
-    syn_brick* d_bricks = (syn_brick*)ctx->ws(nm, sizeof(syn_brick) * (size_t)nbr);
-    if (!d_bricks)
-      return OutOfMemory;
-    cudaMemcpyAsync(d_bricks, hb.data(), sizeof(syn_brick) * (size_t)nbr, cudaMemcpyHostToDevice, st);
     syn_args<T> a;
     memset(&a, 0, sizeof a);
-    a.nbricks = nbr;
+    a.nbricks = sl.nb[0] * sl.nb[1] * sl.nb[2] * nbatch;
     a.coarsest = l + 1 == L;
     a.finest = l == 0;
     a.norm_mask = sl.norm_mask;
     memcpy(a.inv_weight, sl.inv_weight, sizeof a.inv_weight);
-    a.bricks = d_bricks;
+    memcpy(a.nb, sl.nb, sizeof a.nb);
+    if (l + 1 < L)
+      memcpy(a.npb, lv[(size_t)l + 1].nb, sizeof a.npb);
+    a.cbase = sl.base;
     a.cstride = count;
     a.gstride = gcount;
     a.gdims[0] = f.dims.x;
     a.gdims[1] = f.dims.y;
     a.gdims[2] = f.dims.z;
+    char nm[32];
     snprintf(nm, sizeof nm, "syn.lev%d", step & 1);
     if (!adjoint)
     {
@@ -794,7 +943,7 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
         a.out = (T*)out;
       else
       {
-        a.bricks_out = (T*)ctx->ws(nm, (size_t)nbr * (size_t)NB * sizeof(T));
+        a.bricks_out = (T*)ctx->ws(nm, (size_t)a.nbricks * (size_t)NB * sizeof(T));
         if (!a.bricks_out)
           return OutOfMemory;
       }
@@ -805,26 +954,34 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
       a.out = (T*)out;
       if (l + 1 < L)
       {
-        const size_t pn = (size_t)lv[(size_t)l + 1].bricks.size() * (size_t)nbatch * (size_t)NB;
+        const size_t pn = (size_t)a.npb[0] * (size_t)a.npb[1] * (size_t)a.npb[2] * (size_t)nbatch * (size_t)NB;
         a.pgrad = (T*)ctx->ws(nm, pn * sizeof(T));
         if (!a.pgrad)
           return OutOfMemory;
         cudaMemsetAsync(a.pgrad, 0, pn * sizeof(T), st);
       }
     }
-    cudaEventRecord(ctx->ev0, st);
+    // the levels follow one another on the stream; the host waits once, after the last
+    cudaEvent_t t0 = ctx->ev((size_t)(2 * step)), t1 = ctx->ev((size_t)(2 * step + 1));
+    if (!t0 || !t1)
+      return CudaError;
+    cudaEventRecord(t0, st);
     const int e = f.is2d() ? launch_synth<T, true>(ctx, a, adjoint, st) : launch_synth<T, false>(ctx, a, adjoint, st);
-    cudaEventRecord(ctx->ev1, st);
+    cudaEventRecord(t1, st);
     if (e)
       return e;
     prev = adjoint ? a.pgrad : a.bricks_out;
     ++ctx->launches;
     if (cudaGetLastError() != cudaSuccess)
       return CudaError;
-    if (cudaStreamSynchronize(st) != cudaSuccess)
-      return CudaError;
+  }
+  if (cudaStreamSynchronize(st) != cudaSuccess)
+    return CudaError;
+  float total = 0;
+  for (int step = 0; step < L; ++step)
+  {
     float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+    cudaEventElapsedTime(&ms, ctx->ev((size_t)(2 * step)), ctx->ev((size_t)(2 * step + 1)));
     total += ms;
   }
   if (kernel_ms)

@@ -25,12 +25,14 @@ static uint32_t spread3(uint32_t x)
     r |= ((x >> i) & 1u) << (3 * i);
   return r;
 }
+// every third bit of c, packed (10 bits), by halving the gaps
 static uint32_t compact3(uint32_t c)
 {
-  uint32_t r = 0;
-  for (int i = 0; i < 10; ++i)
-    r |= ((c >> (3 * i)) & 1u) << i;
-  return r;
+  c &= 0x09249249u;
+  c = (c | (c >> 2)) & 0x030c30c3u;
+  c = (c | (c >> 4)) & 0x0300f00fu;
+  c = (c | (c >> 8)) & 0x030000ffu;
+  return (c | (c >> 16)) & 0x3ffu;
 }
 
 void subband_blocks(const dataset_format& f, int level, int sb, std::vector<block_geom>* out)

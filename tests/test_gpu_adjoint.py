@@ -189,3 +189,27 @@ def test_differentiable_decode_at_workload_sizes(idx2g, tmp_path):
         c0[i] = old
         fd = float(torch.sum((xp - target[0]) ** 2 - (xm - target[0]) ** 2)) / x.numel() / (2 * h)
         assert abs(fd - float(grad[i])) <= 1e-6 * abs(fd) + 1e-14, (i, fd, float(grad[i]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,levels", [((129, 130, 160), 3), ((33, 64, 97), 1), ((65, 95, 128), 2)])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_synth_batch_and_gradient_at_edges(idx2g, dims, levels, dtype):
+    """Bricks of 1, 2, 31 and 32 valid samples per axis, one to three levels, two fields in a call:
+    the grid and the gradient against the FP64 reference (the bounds of the tests above)."""
+    import torch
+    from idx2_b200.diff import Format, coeff_count, synth, synth_adjoint
+    fmt = Format(dims, dtype, levels)
+    td = torch.float64 if dtype == "float64" else torch.float32
+    n = coeff_count(fmt)
+    c = torch.stack([_coeffs(n, 11 + i, td) for i in range(2)])
+    g = torch.stack([_coeffs(int(np.prod(dims)), 21 + i, td).reshape(fmt.shape) for i in range(2)])
+    grid, grad = synth(c, fmt), synth_adjoint(g, fmt)
+    bound = 1e-10 if dtype == "float64" else 1e-5
+    for i in range(2):
+        cr = c[i].double().cpu().requires_grad_(True)
+        want = ref.synth(cr, dims, levels)
+        (want_grad,) = torch.autograd.grad(want, cr, g[i].double().cpu())
+        want = want.detach()
+        assert float((grid[i].double().cpu() - want).norm() / want.norm()) <= bound
+        assert float((grad[i].double().cpu() - want_grad).norm() / want_grad.norm()) <= bound
