@@ -7,6 +7,7 @@
 #include "dpack_device.h"
 #include "encoder.h"
 #include "format.h"
+#include "host_copy.h"
 #include "shard.h"
 #include "trace.h"
 
@@ -210,13 +211,10 @@ IDX2G_API int idx2g_encode(idx2g_ctx* c, const idx2g_params* in, const void* fie
     void* staged = c->d.ws("enc.field", bytes);
     if (!staged)
       return OutOfMemory;
-    cudaPointerAttributes pa;
-    const bool pinned = cudaPointerGetAttributes(&pa, field) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-    cudaGetLastError();
-    if (pinned && p.dims.z > 1 && c->d.copies())
+    if (is_pinned(field) && p.dims.z > 1 && c->d.copies())
       host_field = field;
-    else
-      cudaMemcpyAsync(staged, field, bytes, cudaMemcpyHostToDevice, c->d.stream);
+    else if (const int ce = host_copy(&c->d, staged, field, bytes, false, c->d.stream))
+      return ce;
     d_field = staged;
   }
   encode_timing tm;
@@ -516,7 +514,8 @@ IDX2G_API int idx2g_encode_batch(idx2g_ctx* c, const idx2g_params* in, const voi
     for (int i = 0; i < n; ++i)
     {
       const size_t b = (size_t)prod(ps[(size_t)i].dims) * (ps[(size_t)i].type == dtype::float32 ? 4 : 8);
-      cudaMemcpyAsync(staged + at, fields[i], b, cudaMemcpyHostToDevice, st);
+      if (const int ce = host_copy(&c->d, staged + at, fields[i], b, false, st))
+        return ce;
       dptr[(size_t)i] = staged + at;
       at += (b + 255) & ~(size_t)255;
     }

@@ -13,6 +13,7 @@
 //   5  keep the brick for the next level, or crop + cast it into the output grid.
 #include "codec_device.cuh"
 #include "decode_device.h"
+#include "host_copy.h"
 #include "trace.h"
 
 #include <algorithm>
@@ -1078,7 +1079,8 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
     {
       for (size_t i = 0; i < n; ++i)
         if (out_bytes[i])
-          cudaMemcpyAsync(outs[i], d_out[i], out_bytes[i], cudaMemcpyDeviceToHost, st);
+          if (const int e = host_copy(ctx, outs[i], d_out[i], out_bytes[i], true, st))
+            return e;
       if (cudaStreamSynchronize(st) != cudaSuccess)
         return CudaError;
     }
