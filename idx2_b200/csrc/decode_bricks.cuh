@@ -27,16 +27,20 @@
 // Kept bricks are stored x fastest, 33^3 doubles, in natural order.
 //
 // Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
-// 7.4 ms against 28.3 ms with k_decode_level; one brick per CTA (8 bricks) 59 against 184 us. At
-// 512^3 57 K warp instructions per brick (354 K before), 26% issue activity: what is left is the
-// latency of the L2 round trips at 16 warps per SM (128 registers a thread).
+// 28.3 ms with k_decode_level, 6.2 ms now; one brick per CTA (8 bricks) 184 and 54 us. At
+// 512^3 57 K warp instructions per brick (354 K before), 26% issue activity: what is left is
+// latency at 16 warps per SM (128 registers a thread, 99 KB of shared memory per CTA). Not kept,
+// as no faster: the next brick's parameters, exponents and tables fetched ahead (13% slower: more
+// of the slots leave L2), plane words as 32-byte loads or marked evict-first, the next task's
+// blocks looked up ahead, one CTA of 16 warps per SM in large launches.
 #pragma once
 
 constexpr int kFaceRow = 33;
 constexpr int kFace = 33 * 33;
 // A z-plane in a slot: four parity classes (hx, hy), each of rows of 17 samples: sample (x, y) at
 // slot_xy(x, y). Rows of one class are read and written 16 lanes at a time, contiguous.
-constexpr int kSlotPlane = 2 * 17 * 33;
+// (1,122 of them, padded to whole lines of 128 bytes)
+constexpr int kSlotPlane = 1136;
 constexpr int kSlotBrick = 33 * kSlotPlane;
 // A warp's tile buffer: z sample (16 of even z, then 16 of odd z) major, 64 columns, the row
 // padded to 65 words: lanes store with (tile, z block, parity) -> banks t + 4 zb + 16 hz.
@@ -60,6 +64,7 @@ struct brick_smem
   double scale[W][32];    // dequantisation of the task's blocks, by lane
   uint8_t block[8][128];       // block of (zb * 5 + yb) * 5 + xb in the subband's walk, 255: not coded
   decode_target rq;
+  decode_brick br;
   int sig;
 };
 static_assert(sizeof(brick_smem<1>::w[0]) % 16 == 0, "every warp's rows start 16-byte aligned");
@@ -574,17 +579,21 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
   }
   for (int bi = blockIdx.x; bi < a.nbricks; bi += gridDim.x)
   {
-    const decode_brick& br = a.bricks[bi];
+    // the brick's and its request's parameters to shared memory: read all through the brick,
+    // between stores that would have them loaded from global memory again each time
     {
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(a.reqs + br.req);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.rq);
-      for (int i = tid; i < (int)(sizeof(decode_target) / 4); i += 32 * W)
-        dst[i] = src[i];
+      static_assert(sizeof(decode_brick) % 4 == 0 && sizeof(decode_target) % 4 == 0, "copied as words");
+      constexpr int nb = (int)(sizeof(decode_brick) / 4), nr = (int)(sizeof(decode_target) / 4);
+      if (tid < nb)
+        reinterpret_cast<uint32_t*>(&sm.br)[tid] = reinterpret_cast<const uint32_t*>(a.bricks + bi)[tid];
+      for (int i = tid - 64; i >= 0 && i < nr; i += 32 * W)
+        reinterpret_cast<uint32_t*>(&sm.rq)[i] = reinterpret_cast<const uint32_t*>(a.reqs + a.bricks[bi].req)[i];
     }
     if (tid == 0)
       sm.sig = 0;
     __syncthreads();
     const decode_target& rq = sm.rq;
+    const decode_brick& br = sm.br;
     // 1: the faces
     if (warp < 7)
       rebuild_face(a, sm, br, bi, warp, lane, sig_level);
@@ -615,10 +624,21 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
     const bool vec4 = a.out_f32 && rq.is_output && br.dims[0] == 32 && br.src_from[0] == 0 && br.src_strd[0] == 1 &&
                       br.dst_strd[0] == 1 && br.dst_from[0] % 4 == 0 && rq.out_dims[0] % 4 == 0 &&
                       (reinterpret_cast<uintptr_t>(rq.out) & 15) == 0;
-    const int nplanes = rq.is_output ? br.dims[2] : 33;
+    const bool output = rq.is_output != 0;
+    const int nplanes = output ? br.dims[2] : 33;
+    // row r of output plane p goes to out0 + p * out_z + r * out_y (elements), from row
+    // src_y + r * src_sy of the brick's plane src_z + p * src_sz
+    const int nx = br.dims[0], ny = br.dims[1];
+    const int src_y = br.src_from[1], src_sy = br.src_strd[1];
+    const int src_z = br.src_from[2], src_sz = br.src_strd[2];
+    const long long row_n = rq.out_dims[0], plane_n = row_n * rq.out_dims[1];
+    const long long out_y = br.dst_strd[1] * row_n, out_z = br.dst_strd[2] * plane_n;
+    const long long out0 = br.dst_from[2] * plane_n + br.dst_from[1] * row_n + br.dst_from[0];
+    const int src_x = br.src_from[0] + lane * br.src_strd[0];
+    const long long dst_x = (long long)lane * br.dst_strd[0];
     for (int p = warp; p < nplanes; p += W)
     {
-      const int z = rq.is_output ? br.src_from[2] + p * br.src_strd[2] : p;
+      const int z = output ? src_z + p * src_sz : p;
       const double* const S = F + (size_t)z * kSlotPlane;
       double* const T = sm.w[warp].plane;
       {
@@ -630,15 +650,22 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
 #pragma unroll
         for (int y = 0; y < 33; ++y)
           v[y] = c[(y & 1) * (17 * 17) + (y >> 1) * 17];
-        ilift33(v);
-#pragma unroll
-        for (int y = 0; y < 33; ++y)
-          T[y * 33 + lane] = v[y];
+        // (column 32 is waited for with the others: left to the compiler its loads went after the
+        // lift and a second round trip to L2; 1024^3 13.9 -> 13.3 ms)
+        asm volatile("" : "+d"(e), "+d"(o));
         ilift33_lanes(e, o, lane);
         if (lane < 17)
           T[2 * lane * 33 + 32] = e;
         if (lane < 16)
           T[(2 * lane + 1) * 33 + 32] = o;
+        ilift33(v);
+#pragma unroll
+        for (int y = 0; y < 33; ++y)
+          T[y * 33 + lane] = v[y];
+        // the plane is done with: its lines need not go to memory (1024^3: 13.9 against 14.3 ms)
+        __syncwarp();
+        for (int k = lane; k < kSlotPlane / 16; k += 32)
+          asm volatile("discard.global.L2 [%0], 128;\n" ::"l"(S + 16 * k) : "memory");
       }
       __syncwarp();
       double v[33];
@@ -646,7 +673,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
       for (int x = 0; x < 33; ++x)
         v[x] = T[lane * 33 + x];
       ilift33(v);
-      if (!rq.is_output)
+      if (!output)
       {
         double e = lane < 17 ? T[32 * 33 + 2 * lane] : 0.0;
         double o = lane < 16 ? T[32 * 33 + 2 * lane + 1] : 0.0;
@@ -666,8 +693,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
       }
       else
       {
-        const long long oz = br.dst_from[2] + (long long)p * br.dst_strd[2];
-        const long long zbase = oz * rq.out_dims[1] * (long long)rq.out_dims[0] + br.dst_from[0];
+        const long long at = out0 + p * out_z;
         __syncwarp();
         if (vec4)
         {
@@ -678,13 +704,14 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
               make_float4(__double2float_rn(v[x]), __double2float_rn(v[x + 1]), __double2float_rn(v[x + 2]),
                           __double2float_rn(v[x + 3]));
           __syncwarp();
-          for (int r = lane >> 3; r < br.dims[1]; r += 4)
-          {
-            const int y = br.src_from[1] + r * br.src_strd[1];
-            const long long oy = br.dst_from[1] + (long long)r * br.dst_strd[1];
-            __stcs(reinterpret_cast<float4*>((float*)rq.out + zbase + oy * rq.out_dims[0]) + (lane & 7),
-                   *(reinterpret_cast<const float4*>(R + y * 36) + (lane & 7)));
-          }
+          // 4 rows at a time, 8 lanes each
+          const float* r0 = R + (src_y + (lane >> 3) * src_sy) * 36 + 4 * (lane & 7);
+          float* g = (float*)rq.out + at + (lane >> 3) * out_y + 4 * (lane & 7);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (4 * k + (lane >> 3) < ny)
+              __stcs(reinterpret_cast<float4*>(g + 4 * k * out_y),
+                     *reinterpret_cast<const float4*>(r0 + 4 * k * src_sy * 36));
         }
         else
         {
@@ -692,16 +719,23 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_decode_bricks(const dec_args
           for (int x = 0; x < 33; ++x)
             T[lane * 33 + x] = v[x];
           __syncwarp();
-          const int sx = br.src_from[0] + lane * br.src_strd[0];
-          for (int r = 0; r < br.dims[1] && lane < br.dims[0]; ++r)
+          if (lane < nx)
           {
-            const int y = br.src_from[1] + r * br.src_strd[1];
-            const long long oy = br.dst_from[1] + (long long)r * br.dst_strd[1];
-            const long long di = zbase + oy * rq.out_dims[0] + (long long)lane * br.dst_strd[0];
+            const double* r0 = T + src_y * 33 + src_x;
             if (a.out_f32)
-              ((float*)rq.out)[di] = __double2float_rn(T[y * 33 + sx]);
+            {
+              float* g = (float*)rq.out + at + dst_x;
+#pragma unroll 8
+              for (int r = 0; r < ny; ++r)
+                __stcs(g + r * out_y, __double2float_rn(r0[r * src_sy * 33]));
+            }
             else
-              ((double*)rq.out)[di] = T[y * 33 + sx];
+            {
+              double* g = (double*)rq.out + at + dst_x;
+#pragma unroll 8
+              for (int r = 0; r < ny; ++r)
+                __stcs(g + r * out_y, r0[r * src_sy * 33]);
+            }
           }
         }
       }

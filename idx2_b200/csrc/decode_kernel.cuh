@@ -591,10 +591,10 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, Pu
 // the run must end.
 //
 // Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
-// 6.5 ms against 9.5 ms with 64-bit windows refilled from global memory where they ran out (6.8
-// ms with the bit scan alone); 64 units, where only the chain counts, 124 against 350 us (145).
-// What bounds it is instructions: 74% issue activity with 9 of 32 lanes active, as every step
-// waits for its longest plane.
+// 6.65 ms against 9.5 ms with 64-bit windows refilled from global memory where they ran out; 64
+// units, where only the chain counts, 104 against 350 us (145 with the bit scan alone, 124 with
+// the table and the bit scan on different sides of a branch). What bounds it is instructions: 158 K
+// per brick at 74% issue activity, 9 of 32 lanes active, as every step waits for its longest plane.
 // ---------------------------------------------------------------------------
 constexpr int kRingWords = 16;
 constexpr unsigned kRingMask = (kRingWords - 1) * 128;  // byte offset of a ring word, 32 lanes wide
@@ -662,47 +662,42 @@ __device__ __forceinline__ uint32_t ring_peek(const uint32_t* ring, uint32_t p)
   return __funnelshift_r(lo, hi, p);
 }
 
-// One bit plane (Core/Zfp.h:990 Decode<u64>) from position p: at most 128 bits. The plane's bits
-// in (xlo, xhi); n (significant coefficients) and p advance.
-__device__ __forceinline__ void ring_plane(const uint32_t* ring, const uint16_t* tests, uint32_t& p, int& n, int nvals,
-                                           uint32_t& xlo, uint32_t& xhi)
+// One bit plane (Core/Zfp.h:990 Decode<u64>) of a block with n significant coefficients, from
+// position p (at most 128 bits): raw holds the 64 bits from p on. The plane's bits in (xlo, xhi);
+// n and p advance.
+__device__ __forceinline__ void ring_plane(const uint32_t* ring, const uint16_t* tests, uint32_t rawlo, uint32_t rawhi,
+                                           uint32_t& p, int& n, int nvals, uint32_t& xlo, uint32_t& xhi)
 {
-  xlo = 0;
-  xhi = 0;
-  if (n > 0)
-  {
-    xlo = ring_peek(ring, p) & ~shl_to0(~0u, n);
-    if (n > 32)
-      xhi = ring_peek(ring, p + 32) & ~shl_to0(~0u, n - 32);
-    p += (uint32_t)n;
-  }
-  if (n >= nvals)
-    return;
+  xlo = rawlo & ~shl_to0(~0u, n);
+  xhi = rawhi & ~shl_to0(~0u, n > 32 ? n - 32 : 0);
+  p += (uint32_t)n;
   const int last = nvals - 1;
-  do
+  while (n < nvals)
   {
     const uint32_t g = ring_peek(ring, p);
     const uint32_t e = tests[g & ((1u << kTestBits) - 1u)];
     // coefficients before the last one (the last one's run has no end bit)
     const int lim = last - n;
-    const uint32_t found = e & (kTestsEnd - 1u), take = found & ~shl_to0(~0u, lim);
-    if (take == 0 && e != kTestsEnd)
+    const uint32_t found = e & (kTestsEnd - 1u);
+    uint32_t take = found & ~shl_to0(~0u, lim);
+    const bool one = take == 0 && e != kTestsEnd;
+    // one: a test and its run that the table does not hold (or the last coefficient's), up to the
+    // next significant coefficient, or the last one
+    const uint32_t h = (g >> 1) | shl_to0(1u, lim);
+    const bool end = e >= kTestsEnd && take == found;
+    take = one ? h & (0u - h) : take;
+    if (one && h == 0)
     {
-      // one test and its run, which the table does not hold (or the last coefficient's): up to
-      // the next significant coefficient, or the last one
-      const uint32_t h = (g >> 1) | shl_to0(1u, lim);
-      int z = __ffs((int)h) - 1;
-      if (h == 0)
-      {
-        const uint32_t lo = ring_peek(ring, p + 32), hi = ring_peek(ring, p + 64);
-        z = lo ? 30 + __ffs((int)lo) : (hi ? 62 + __ffs((int)hi) : 64);
-        z = z < lim ? z : lim;
-      }
+      // a run of more than 31
+      const uint32_t lo = ring_peek(ring, p + 32), hi = ring_peek(ring, p + 64);
+      int z = lo ? 30 + __ffs((int)lo) : (hi ? 62 + __ffs((int)hi) : 64);
+      z = z < lim ? z : lim;
       n += z;
       p += (uint32_t)(z + 2);
       xlo |= shl_to0(1u, n);
       xhi |= shl_to0(1u, n - 32);
       ++n;
+      p -= n == nvals ? 1u : 0u;  // (the last run has no end bit)
       continue;
     }
     xlo |= shl_to0(take, n);
@@ -710,14 +705,13 @@ __device__ __forceinline__ void ring_plane(const uint32_t* ring, const uint16_t*
     const int a = 32 - __clz((int)take);
     n += a;
     p += (uint32_t)(a + __popc(take));
-    if (e >= kTestsEnd && take == found)
+    if (end)
     {
       ++p;
       return;
     }
-  } while (n < nvals);
-  if (n == nvals)
-    --p;  // the last run has no end bit
+    p -= n == nvals ? 1u : 0u;
+  }
 }
 
 struct ring_smem
@@ -778,6 +772,7 @@ __device__ __forceinline__ void plane_wavefront_ring(const dec1_args& a, const p
     }
   }
   unsigned long long* row = U.T - (long long)c * U.stride;
+  uint32_t w_next = c == 0 ? info[0] : 0u;  // the block of the next step, loaded a step ahead
   int st = 0;  // significant coefficients after the lane's last plane, 256: the block's planes have ended
   for (int t = 0; t < steps; ++t, row += U.stride)
   {
@@ -789,25 +784,24 @@ __device__ __forceinline__ void plane_wavefront_ring(const dec1_args& a, const p
       put();
     if (has && loaded - (int)(p >> 5) <= kRingWords - 4)
       fetch();
+    const uint32_t rawlo = ring_peek(ring, p), rawhi = ring_peek(ring, p + 32);
     const int b = t - c;
+    const uint32_t w = w_next;
+    w_next = (unsigned)(b + 1) < (unsigned)nb ? info[b + 1] : 0u;
     st = 0;
-    if (c < nkeys && (unsigned)b < (unsigned)nb)
+    const int kk = (int)(w & 0xffffu) - key;
+    if (c < nkeys && (unsigned)kk < ((w >> 16) & 0xffu))
     {
-      const uint32_t w = info[b];
-      const int kk = (int)(w & 0xffffu) - key;
-      if ((unsigned)kk < ((w >> 16) & 0xffu))
+      int n = kk == 0 ? 0 : in & 255;
+      uint32_t xlo = 0, xhi = 0;
+      if (!has || (kk != 0 && in >= 256))
+        st = n | 256;
+      else
       {
-        int n = kk == 0 ? 0 : in & 255;
-        uint32_t xlo = 0, xhi = 0;
-        if (!has || (kk != 0 && in >= 256))
-          st = n | 256;
-        else
-        {
-          ring_plane(ring, tests, p, n, 1 << (w >> 24), xlo, xhi);
-          st = n;
-        }
-        row[kk] = ((unsigned long long)xhi << 32) | xlo;
+        ring_plane(ring, tests, rawlo, rawhi, p, n, 1 << (w >> 24), xlo, xhi);
+        st = n;
       }
+      row[kk] = ((unsigned long long)xhi << 32) | xlo;
     }
   }
 }
