@@ -335,40 +335,53 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_ranks(const dpack_args a)
 }
 
 // ---------------------------------------------------------------------------
-// per segment: raw exponents, and a warp per chunk writing its header and data
+// raw exponents (Core/idx2Encode.cpp:41 EncodeBrickSubbandExponents): EMax + 127 as a byte
+// (float32) or EMax + 1023 as a little-endian 16-bit word (float64), events in order; a warp per
+// event. A kernel of its own ahead of the key pass: the host compresses the exponents (1.7 ms for
+// 384x384x256 float64) while the device packs, instead of after it.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kPackThreads) k_pack_exps(const dpack_args a)
+{
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * kPackThreads + (int)threadIdx.x) >> 5; i < a.nev; i += (gridDim.x * kPackThreads) >> 5)
+  {
+    const dpack_event& e = a.evs[i];
+    const dpack_segment& S = a.segs[e.seg];
+    const region_dev r = region_of(a, S, e);
+    uint8_t* dst = a.exps + S.exp_off + (size_t)(i - S.ev0) * (size_t)S.nexps * (size_t)a.exp_bytes;
+    for (int b = lane; b < S.nexps; b += 32)
+    {
+      const int v = r.exps[b];
+      if (a.exp_bytes == 1)
+        dst[b] = (uint8_t)(v + 127);
+      else
+      {
+        const uint16_t u = (uint16_t)(v + 1023);
+        dst[2 * b] = (uint8_t)(u & 0xFF);
+        dst[2 * b + 1] = (uint8_t)(u >> 8);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// a warp per key of a sub-range writing its part of the chunk's header and data. The keys of a
+// sub-range are spread over gridDim.y CTAs: a warp walks a key's 256 events one after the other,
+// and with one CTA per sub-range a dataset of few sub-ranges left the device idle (48 of them,
+// 384x384x256 float64: 405 us, 237 us with 8 CTAs each).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kPackThreads) k_pack_write(const dpack_args a)
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // a CTA per sub-range of a segment, a warp per key
   for (int ci = blockIdx.x; ci < a.nsub; ci += gridDim.x)
   {
     const int4 sr = a.subs[ci];
     const int si = sr.x;
     const dpack_segment& S = a.segs[si];
-    // raw exponents (Core/idx2Encode.cpp:41 EncodeBrickSubbandExponents): EMax + 127 as a
-    // byte (float32) or EMax + 1023 as a little-endian 16-bit word (float64), events in order
-    for (int i = sr.y + warp; i < sr.z; i += kPackWarps)
-    {
-      const region_dev r = region_of(a, S, a.evs[i]);
-      uint8_t* dst = a.exps + S.exp_off + (size_t)(i - S.ev0) * (size_t)S.nexps * (size_t)a.exp_bytes;
-      for (int b = lane; b < S.nexps; b += 32)
-      {
-        const int v = r.exps[b];
-        if (a.exp_bytes == 1)
-          dst[b] = (uint8_t)(v + 127);
-        else
-        {
-          const uint16_t u = (uint16_t)(v + 1023);
-          dst[2 * b] = (uint8_t)(u & 0xFF);
-          dst[2 * b + 1] = (uint8_t)(u >> 8);
-        }
-      }
-    }
     const int K0 = a.seg_kmin[si];
     if (K0 == 0x7fffffff)
       continue;
-    for (int k = warp; k < kSegKeys; k += kPackWarps)
+    for (int k = warp + (int)blockIdx.y * kPackWarps; k < kSegKeys; k += kPackWarps * (int)gridDim.y)
     {
       const dpack_key rec = a.keys[(size_t)si * kSegKeys + k];
       if (!rec.n)
@@ -484,11 +497,20 @@ void dpack_launch_keys(const dpack_args& a, int grid, cudaStream_t st)
   k_pack_ranks<<<grid, kPackThreads, 0, st>>>(a);
 }
 
-void dpack_launch_write(const dpack_args& a, int grid, cudaStream_t st)
+void dpack_launch_exps(const dpack_args& a, cudaStream_t st)
 {
-  (void)grid;
-  const int sgrid = a.nsub < 65535 ? a.nsub : 65535;
-  k_pack_write<<<sgrid > 0 ? sgrid : 1, kPackThreads, 0, st>>>(a);
+  const int eg = (a.nev + kPackWarps - 1) / kPackWarps;
+  k_pack_exps<<<eg < 1 ? 1 : (eg < 65535 ? eg : 65535), kPackThreads, 0, st>>>(a);
+}
+
+void dpack_launch_write(const dpack_args& a, int num_sms, cudaStream_t st)
+{
+  const int sgrid = a.nsub < 65535 ? (a.nsub > 0 ? a.nsub : 1) : 65535;
+  // enough CTAs to fill the device (8 per SM), at most 8 per sub-range: 64 keys, more than a
+  // sub-range usually has
+  int per = (8 * num_sms + sgrid - 1) / sgrid;
+  per = per < 2 ? 2 : (per > 8 ? 8 : per);
+  k_pack_write<<<dim3((unsigned)sgrid, (unsigned)per), kPackThreads, 0, st>>>(a);
 }
 
 } // namespace idx2g

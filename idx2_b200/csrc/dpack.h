@@ -114,9 +114,12 @@ struct dpack_layout
 // files' chunk tables (sizes, addresses) and the bit-plane statistics.
 int dpack_make_layout(const dataset_format& f, const dpack_plan& P, const std::vector<dpack_key>& keys,
                       const std::vector<int>& kmin, dpack_layout* L, packed_dataset* out);
+// The zstd frame of every segment's raw exponents (host copy), on several threads.
+int dpack_compress(const dpack_plan& P, const uint8_t* exps, std::vector<std::vector<uint8_t>>* frames);
 // From k_pack_write's output (host copies of the image and of the raw exponents): exponent
-// chunks (zstd), file contents and tails, the remaining statistics.
+// chunks (frames: dpack_compress's, made here when null), file contents and tails, the remaining
+// statistics.
 int dpack_finish(const dataset_format& f, const dpack_plan& P, const dpack_layout& L, const uint8_t* image,
-                 const uint8_t* exps, packed_dataset* out);
+                 const uint8_t* exps, packed_dataset* out, std::vector<std::vector<uint8_t>>* frames = nullptr);
 
 } // namespace idx2g

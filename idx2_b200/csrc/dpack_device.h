@@ -66,8 +66,9 @@ struct dpack_args
   int* error;                        // 1: a segment spans more than kSegKeys keys, 2: kb too small
 };
 
+void dpack_launch_exps(const dpack_args& a, cudaStream_t st);
 void dpack_launch_keys(const dpack_args& a, int grid, cudaStream_t st);
-void dpack_launch_write(const dpack_args& a, int grid, cudaStream_t st);
+void dpack_launch_write(const dpack_args& a, int num_sms, cudaStream_t st);
 
 // Packs the levels' regions on ctx's device. Returns NoError, or NotApplicable when a segment
 // holds more keys than the kernels' window (the caller then packs on the host).

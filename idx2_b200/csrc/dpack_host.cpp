@@ -8,6 +8,7 @@
 #include <chrono>
 #include <cstring>
 #include <fcntl.h>
+#include <system_error>
 #include <thread>
 #include <unistd.h>
 
@@ -140,10 +141,47 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
   a.chunk_off = d_coff;
   a.exps = d_exps;
   a.error = d_err;
+  // the raw exponents first: a thread compresses them while the device packs
+  uint8_t* h_exps = (uint8_t*)ctx->pinned("dpack.hexps", (size_t)P.exp_total + 16);
+  const cudaEvent_t ex = ctx->ev(0);
+  if (!h_exps || !ex)
+    return OutOfMemory;
+  if (P.exp_total)
+  {
+    dpack_launch_exps(a, st);
+    ctx->launches += 1;
+    cudaMemcpyAsync(h_exps, d_exps, (size_t)P.exp_total, cudaMemcpyDeviceToHost, st);
+  }
+  if (cudaEventRecord(ex, st) != cudaSuccess)
+    return CudaError;
+  std::vector<std::vector<uint8_t>> frames;
+  int frames_err = NoError;
+  std::thread compress;
+  struct compress_joiner
+  {
+    std::thread& t;
+    ~compress_joiner()
+    {
+      if (t.joinable())
+        t.join();
+    }
+  } join_compress{ compress };
+  auto make_frames = [&frames, &frames_err, &P, h_exps, ex, dev = ctx->device]() {
+    frames_err = cudaSetDevice(dev) == cudaSuccess && cudaEventSynchronize(ex) == cudaSuccess
+                   ? dpack_compress(P, h_exps, &frames)
+                   : CudaError;
+  };
+  try
+  {
+    compress = std::thread(make_frames);
+  }
+  catch (const std::system_error&)
+  {
+    // no thread to be had: compressed below, after the packing
+  }
   // the key pass (a warp per event, a CTA per sub-range for the totals, a CTA per segment for
-  // the ranks); k_pack_write: a CTA per sub-range
+  // the ranks); k_pack_write: a warp per key of a sub-range
   const int grid = nseg < 4 * ctx->num_sms ? nseg : 4 * ctx->num_sms;
-  const int wgrid = nseg < 2048 ? nseg : 2048;
   dpack_launch_keys(a, grid, st);
   ctx->launches += 4;
   std::vector<dpack_key> keys((size_t)nseg * kSegKeys);
@@ -167,21 +205,13 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
   const size_t img_words = (size_t)((L.total + 3) / 4) + 1;
   uint32_t* d_img = (uint32_t*)ctx->ws("dpack.image", img_words * 4);
   uint8_t* h_img = (uint8_t*)ctx->pinned("dpack.himage", (size_t)L.total + 16);
-  uint8_t* h_exps = (uint8_t*)ctx->pinned("dpack.hexps", (size_t)P.exp_total + 16);
-  if (!d_img || !h_img || !h_exps)
+  if (!d_img || !h_img)
     return OutOfMemory;
   cudaMemcpyAsync(d_coff, L.chunk_off.data(), 8 * L.chunk_off.size(), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(d_img, 0, img_words * 4, st);
   a.image = d_img;
-  dpack_launch_write(a, wgrid, st);
+  dpack_launch_write(a, ctx->num_sms, st);
   ctx->launches += 1;
-  // the raw exponents first: their compression (and the file tails) run on the host while
-  // the image comes back
-  if (P.exp_total)
-    cudaMemcpyAsync(h_exps, d_exps, (size_t)P.exp_total, cudaMemcpyDeviceToHost, st);
-  cudaEvent_t ex = ctx->ev(0);
-  if (!ex || cudaEventRecord(ex, st) != cudaSuccess)
-    return CudaError;
   // the image in pieces, each with an event: the file writer starts on the first pieces
   // while the later ones are still on their way
   constexpr unsigned long long kCopyPiece = 32ull << 20;
@@ -209,10 +239,14 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
   out->image = h_img;
   if (on_image)
     on_image(L, h_img, out->ready);  // e.g. the chunk sections written while the rest is made
-  if (cudaEventSynchronize(ex) != cudaSuccess)
-    return CudaError;
+  if (compress.joinable())
+    compress.join();
+  else
+    make_frames();
+  if (frames_err)
+    return frames_err;
   tt.lap("dpack.write");
-  e = dpack_finish(f, P, L, h_img, h_exps, out);
+  e = dpack_finish(f, P, L, h_img, h_exps, out, &frames);
   tt.lap("dpack.finish");
   return e;
 }

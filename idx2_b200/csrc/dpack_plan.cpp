@@ -261,14 +261,44 @@ int dpack_make_layout(const dataset_format& f, const dpack_plan& P, const std::v
   return NoError;
 }
 
-int dpack_finish(const dataset_format& f, const dpack_plan& P, const dpack_layout& L, const uint8_t* image,
-                 const uint8_t* exps, packed_dataset* out)
+namespace
+{
+
+size_t exp_bytes_of(const dpack_plan& P, int seg)
+{
+  const dpack_segment& s = P.segs[(size_t)seg];
+  return (size_t)(s.ev1 - s.ev0) * (size_t)s.nexps * (size_t)P.exp_bytes;
+}
+
+} // namespace
+
+int dpack_compress(const dpack_plan& P, const uint8_t* exps, std::vector<std::vector<uint8_t>>* frames)
 {
   stage_timer tt;
+  frames->assign(P.segs.size(), std::vector<uint8_t>());
+  std::atomic<int> err{ 0 };
+  parallel_for(P.segs.size(), [&](size_t i) {
+    if (zstd_compress(exps + P.segs[i].exp_off, exp_bytes_of(P, (int)i), &(*frames)[i]))
+      err = UnknownError;
+  });
+  tt.lap("dpack.compress");
+  return err;
+}
+
+int dpack_finish(const dataset_format& f, const dpack_plan& P, const dpack_layout& L, const uint8_t* image,
+                 const uint8_t* exps, packed_dataset* out, std::vector<std::vector<uint8_t>>* frames)
+{
+  stage_timer tt;
+  std::vector<std::vector<uint8_t>> own;
+  if (!frames)
+  {
+    frames = &own;
+    if (const int e = dpack_compress(P, exps, frames))
+      return e;
+  }
   std::map<std::string, file_buffer>& files = out->files;
   pack_stats& stats = out->stats;
   const uint8_t* h_img = image;
-  const uint8_t* h_exps = exps;
   // exponent chunks and their stamps, while the kernel runs: a group writes the exponents
   // it holds at the first brick of each later chunk, and what it holds at the end in the
   // order of FlushChunkExponents (levels descending, then subbands)
@@ -309,37 +339,15 @@ int dpack_finish(const dataset_format& f, const dpack_plan& P, const dpack_layou
     erecs.push_back(r);
   }
   std::sort(erecs.begin(), erecs.end(), [](const exp_rec& x, const exp_rec& y) { return x.st < y.st; });
-  auto raw_of = [&](const exp_rec& r, const uint8_t** p, size_t* n) {
-    if (r.seg < 0)
-    {
-      *p = h_exps;
-      *n = 0;
-      return;
-    }
-    const dpack_segment& s = P.segs[(size_t)r.seg];
-    *p = h_exps + s.exp_off;
-    *n = (size_t)(s.ev1 - s.ev0) * (size_t)s.nexps * (size_t)P.exp_bytes;
-  };
+  // (every segment's exponents are written once, with one of the records; a record without a
+  // segment is empty)
   out->image = h_img;
   out->exps_z.assign(erecs.size(), std::vector<uint8_t>());
-  std::atomic<int> zerr{ 0 };
-  parallel_for(erecs.size(), [&](size_t i) {
-    const uint8_t* p;
-    size_t n;
-    raw_of(erecs[i], &p, &n);
-    if (zstd_compress(p, n, &out->exps_z[i]))
-      zerr = UnknownError;
-  });
-  if (zerr)
-    return zerr;
-  tt.lap("dpack.finish.exps");
   for (size_t i = 0; i < erecs.size(); ++i)
-  {
-    const uint8_t* p;
-    size_t n;
-    raw_of(erecs[i], &p, &n);
-    stats.exp_chunks_raw.add((double)n);
-  }
+    if (erecs[i].seg >= 0)
+      out->exps_z[i] = std::move((*frames)[(size_t)erecs[i].seg]);
+  for (const exp_rec& r : erecs)
+    stats.exp_chunks_raw.add(r.seg < 0 ? 0.0 : (double)exp_bytes_of(P, r.seg));
   for (size_t i = 0; i < erecs.size(); ++i)
   {
     const exp_rec& r = erecs[i];
