@@ -166,6 +166,13 @@ struct enc_smem_t
 };
 using enc_smem = enc_smem_t<kThreads>;
 
+// A z-plane of a 33^3 brick in shared memory (plane_forward, plane_middle): one per warp, as many
+// as the tables' space holds (6 of the 8 warps for float32 data, all of them for float64; a third
+// CTA per SM is worth more than the other two).
+constexpr int kPlaneSamples = 33 * 33;
+constexpr int kPlaneBufs = 6;
+static_assert(kWarps >= 8, "plane buffers belong to warps");
+
 inline size_t enc_smem_bytes(int planes)
 {
   // the coding tables, which also hold the 17^3 even lattice during the transform
@@ -175,6 +182,8 @@ inline size_t enc_smem_bytes(int planes)
   const size_t band = (size_t)kGz * 32 * 32 * (planes == 32 ? 4 : 8) + (size_t)kGz * 33 * 33 * 8;
   size_t space = tables > lattice ? tables : lattice;
   space = space > band ? space : band;
+  const size_t bufs = (size_t)kPlaneBufs * kPlaneSamples * 8;
+  space = space > bufs ? space : bufs;
   return ((sizeof(enc_smem) + 127) & ~(size_t)127) + space;
 }
 
@@ -730,6 +739,154 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
   ENC_PHASE(14)
 }
 
+// One 33-sample line over the lanes of a warp: lane k holds samples 2k (k <= 16) and 2k + 1
+// (k <= 15). The operations of dev::lift_regs, in its order; EXT: a line of 32 samples whose 33rd
+// is extrapolated (forward only).
+template <bool FWD, bool EXT>
+__device__ __forceinline__ void lift_lanes(double& e, double& o, int lane)
+{
+  if constexpr (FWD)
+  {
+    if constexpr (EXT)
+    {
+      const double x = __dsub_rn(__dmul_rn(2.0, __shfl_sync(0xffffffffu, o, 15)), __shfl_sync(0xffffffffu, e, 15));
+      e = lane == 16 ? x : e;
+    }
+    const double r = __shfl_down_sync(0xffffffffu, e, 1);
+    o = __dsub_rn(o, __dmul_rn(__dadd_rn(e, r), 0.5));
+    if (EXT && lane == 15)
+      o = 0.0;
+    const double V = __dmul_rn(o, 0.25), Vl = __shfl_up_sync(0xffffffffu, V, 1);
+    constexpr int last = EXT ? 14 : 15;  // the odd samples that update their neighbours: 0..last
+    if (lane > 0 && lane - 1 <= last)
+      e = __dadd_rn(e, Vl);
+    if (lane <= last)
+      e = __dadd_rn(e, V);
+  }
+  else
+  {
+    const double V = __dmul_rn(o, 0.25), Vl = __shfl_up_sync(0xffffffffu, V, 1);
+    if (lane > 0)
+      e = __dsub_rn(e, Vl);
+    if (lane < 16)
+      e = __dsub_rn(e, V);
+    const double r = __shfl_down_sync(0xffffffffu, e, 1);
+    o = __dadd_rn(o, __dmul_rn(__dadd_rn(e, r), 0.5));
+  }
+}
+
+// The sweeps that stay inside z-planes, a plane per warp and no barrier of the CTA: a lane per
+// row for X, a lane per column for Y (their 33rd over the lanes), the plane turned in the warp's
+// buffer T. Level 0 of a 1024^3 float32 field at 1e-3: 38.1 ms, against 46.2 ms with the CTA sweeping
+// bands of 4 planes between barriers (gpu__time_duration).
+//
+// plane_forward: the first two sweeps (X, then Y) of the extrapolation of a brick with 32 valid
+// samples per axis, from the samples at src (row stride sy) to plane z of the brick.
+template <typename S, bool RANGE>
+__device__ __forceinline__ void plane_forward(const S* src, long long sy, double* T, double* dst, double& mn,
+                                              double& mx, int lane)
+{
+  S* const raw = reinterpret_cast<S*>(T);
+#pragma unroll 8
+  for (int y = 0; y < 32; ++y)
+    raw[y * 33 + lane] = __ldcs(src + (long long)y * sy + lane);
+  __syncwarp();
+  double v[33];
+#pragma unroll
+  for (int x = 0; x < 32; ++x)
+    v[x] = (double)raw[lane * 33 + x];
+  if constexpr (RANGE)
+  {
+#pragma unroll
+    for (int x = 0; x < 32; ++x)
+    {
+      mn = v[x] < mn ? v[x] : mn;
+      mx = mx < v[x] ? v[x] : mx;
+    }
+  }
+  v[32] = 0.0;
+  dev::lift_regs<true>(v, 32);
+  __syncwarp();
+#pragma unroll
+  for (int x = 0; x < 33; ++x)
+    T[lane * 33 + x] = v[x];
+  __syncwarp();
+  double e = T[2 * (lane < 15 ? lane : 15) * 33 + 32], o = T[(2 * (lane < 15 ? lane : 15) + 1) * 33 + 32];
+  lift_lanes<true, true>(e, o, lane);
+  if (lane < 17)
+    dst[2 * lane * 33 + 32] = e;
+  if (lane < 16)
+    dst[(2 * lane + 1) * 33 + 32] = o;
+#pragma unroll
+  for (int y = 0; y < 32; ++y)
+    v[y] = T[y * 33 + lane];
+  v[32] = 0.0;
+  dev::lift_regs<true>(v, 32);
+#pragma unroll
+  for (int y = 0; y < 33; ++y)
+    dst[y * 33 + lane] = v[y];
+  __syncwarp();
+}
+
+// plane_middle: the inverse Y and X sweeps that end the extrapolation and the forward X and Y
+// sweeps of the real transform (Core/Wavelet.cpp:81), on the 33 x 33 plane at P.
+__device__ __forceinline__ void plane_middle(double* P, double* T, int lane)
+{
+  double v[33];
+  {
+    double e = P[2 * (lane < 16 ? lane : 16) * 33 + 32], o = P[(2 * (lane < 15 ? lane : 15) + 1) * 33 + 32];
+#pragma unroll
+    for (int y = 0; y < 33; ++y)
+      v[y] = P[y * 33 + lane];
+    asm volatile("" : "+d"(e), "+d"(o));  // (waited for with the other columns)
+    lift_lanes<false, false>(e, o, lane);
+    if (lane < 17)
+      T[2 * lane * 33 + 32] = e;
+    if (lane < 16)
+      T[(2 * lane + 1) * 33 + 32] = o;
+  }
+  dev::lift_regs<false>(v, 33);
+#pragma unroll
+  for (int y = 0; y < 33; ++y)
+    T[y * 33 + lane] = v[y];
+  __syncwarp();
+  {
+    double e = T[32 * 33 + 2 * (lane < 16 ? lane : 16)], o = T[32 * 33 + 2 * (lane < 15 ? lane : 15) + 1];
+    lift_lanes<false, false>(e, o, lane);
+    lift_lanes<true, false>(e, o, lane);
+    __syncwarp();
+    if (lane < 17)
+      T[32 * 33 + 2 * lane] = e;
+    if (lane < 16)
+      T[32 * 33 + 2 * lane + 1] = o;
+  }
+#pragma unroll
+  for (int x = 0; x < 33; ++x)
+    v[x] = T[lane * 33 + x];
+  dev::lift_regs<false>(v, 33);
+  dev::lift_regs<true>(v, 33);
+#pragma unroll
+  for (int x = 0; x < 33; ++x)
+    T[lane * 33 + x] = v[x];
+  __syncwarp();
+  {
+    double e = T[2 * (lane < 16 ? lane : 16) * 33 + 32], o = T[(2 * (lane < 15 ? lane : 15) + 1) * 33 + 32];
+    lift_lanes<true, false>(e, o, lane);
+    if (lane < 17)
+      P[2 * lane * 33 + 32] = e;
+    if (lane < 16)
+      P[(2 * lane + 1) * 33 + 32] = o;
+  }
+#pragma unroll
+  for (int y = 0; y < 33; ++y)
+    v[y] = T[y * 33 + lane];
+  dev::lift_regs<true>(v, 33);
+#pragma unroll
+  for (int y = 0; y < 33; ++y)
+    P[y * 33 + lane] = v[y];
+  __syncwarp();
+}
+
 template <int CPS>
 __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a)
 {
@@ -786,9 +943,63 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
     const bool gather_xy = a.level == 0 && fp.tmap != nullptr && !fp.is2d && sm.stack.coarse >= 2 &&
                            sm.stack.axis[0] + sm.stack.axis[1] == 1 && level_one(sm.stack.g[0]) &&
                            level_one(sm.stack.g[1]);
+    // a brick of 32 valid samples per axis whose first sweeps are X, Y and Z: X and Y take a
+    // plane per warp straight from the samples (Z makes the 33rd plane)
+    const bool by_plane = !fp.is2d && br.valid[0] == 32 && br.valid[1] == 32 && br.valid[2] == 32 &&
+                          sm.stack.coarse >= 3 && sm.stack.axis[0] == 0 && sm.stack.axis[1] == 1 &&
+                          sm.stack.axis[2] == 2 && level_one(sm.stack.g[0]) && level_one(sm.stack.g[1]);
+    const int nbufs = P == 32 ? kPlaneBufs : 8;
+    double* const plane_buf = reinterpret_cast<double*>(Xp) + (size_t)warp * kPlaneSamples;
     ENC_PHASE_START
     // ---------------- A: gather ----------------
-    if (a.level == 0 && gather_xy)
+    if (by_plane)
+    {
+      double mn = 1.7976931348623157e308, mx = -1.7976931348623157e308;
+      if (warp < nbufs)
+      {
+        const long long at0 =
+          (((long long)br.b3[2] * 32) * fp.fdims[1] + (long long)br.b3[1] * 32) * fp.fdims[0] + (long long)br.b3[0] * 32;
+        const long long sz = fp.fdims[0] * fp.fdims[1];
+        for (int z = warp; z < 32; z += nbufs)
+        {
+          double* dst = F + (size_t)z * kPlaneSamples;
+          if (a.level > 0)
+            plane_forward<double, false>(a.in_bricks + (size_t)bi * (size_t)kNB3 + (size_t)z * kPlaneSamples, 33,
+                                         plane_buf, dst, mn, mx, lane);
+          else if (fp.field_f32)
+            plane_forward<float, true>((const float*)fp.field + at0 + z * sz, fp.fdims[0], plane_buf, dst, mn, mx, lane);
+          else
+            plane_forward<double, true>((const double*)fp.field + at0 + z * sz, fp.fdims[0], plane_buf, dst, mn, mx,
+                                        lane);
+        }
+      }
+      if (a.level == 0)
+      {
+        for (int o = 16; o > 0; o >>= 1)
+        {
+          double w1 = __shfl_xor_sync(0xffffffffu, mn, o), w2 = __shfl_xor_sync(0xffffffffu, mx, o);
+          mn = w1 < mn ? w1 : mn;
+          mx = mx < w2 ? w2 : mx;
+        }
+        if (lane == 0)
+        {
+          sm.red[0][warp] = mn;
+          sm.red[1][warp] = mx;
+        }
+        __syncthreads();
+        if (tid == 0)
+        {
+          for (int w = 1; w < kWarps; ++w)
+          {
+            mn = sm.red[0][w] < mn ? sm.red[0][w] : mn;
+            mx = mx < sm.red[1][w] ? sm.red[1][w] : mx;
+          }
+          a.bmin[bi] = mn;
+          a.bmax[bi] = mx;
+        }
+      }
+    }
+    else if (a.level == 0 && gather_xy)
     {
       // one chunk buffer: the copy of chunk c + 1 runs while chunk c's sweeps do
       const int vx = br.valid[0], vy = br.valid[1], vz = br.valid[2];
@@ -1092,7 +1303,29 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
       const int NS[3] = { 17, 17, fp.is2d ? 1 : 17 };
       const int nsub = NS[0] * NS[1] * NS[2];
       const int nf = sm.stack.n, cf = sm.stack.coarse;
-      for (int i = gather_xy ? 2 : 0; i < cf; ++i)
+      // A column with x or y odd holds no sample of the lattice: its forward Z sweep is followed by
+      // the inverse one at once (one read and one write of it less; 38.1 -> 37.3 ms at 1024^3).
+      const bool fuse_z = by_plane && cf == 3 && level_one(sm.stack.g[2]);
+      if (fuse_z)
+      {
+        for (int li = tid; li < 33 * 33; li += kThreads)
+        {
+          double* col = F + li;
+          double v[33];
+#pragma unroll
+          for (int k = 0; k < 32; ++k)
+            v[k] = col[k * 33 * 33];
+          v[32] = 0.0;
+          dev::lift_regs<true>(v, 32);
+          if (((li % 33) | (li / 33)) & 1)
+            dev::lift_regs<false>(v, 33);
+#pragma unroll
+          for (int k = 0; k < 33; ++k)
+            col[k * 33 * 33] = v[k];
+        }
+        __syncthreads();
+      }
+      for (int i = fuse_z ? 3 : (gather_xy || by_plane ? 2 : 0); i < cf; ++i)
       {
         dev::lift_sweep_regs<true>(F, N, sm.stack.g[i], sm.stack.axis[i]);
         __syncthreads();
@@ -1132,72 +1365,31 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
       ENC_PHASE(4)
       // With the first level's sweeps in Z, Y, X order on the whole 33^3 brick (the usual
       // transform order), the sweeps that stay inside z-planes -- the inverse Y, the inverse
-      // then forward X, and the forward Y -- run on bands of kPlanes z-planes in shared
-      // memory (the coding tables' space, idle here): one read and one write of the brick
-      // instead of three of each. The same line functions run on the same values.
+      // then forward X, and the forward Y -- take a plane per warp (plane_middle; the buffers are
+      // in the coding tables' space, idle here): one read and one write of the brick instead of
+      // three of each.
       auto full33 = [&](const dev::dgrid& g) {
         return g.from[0] == 0 && g.from[1] == 0 && g.from[2] == 0 && g.dims[0] == 33 && g.dims[1] == 33 &&
                g.dims[2] == 33 && g.strd[0] == 1 && g.strd[1] == 1 && g.strd[2] == 1;
       };
       const bool planar = !fp.is2d && ci == 3 && sm.stack.axis[2] == 2 && sm.stack.axis[1] == 1 &&
                           sm.stack.axis[0] == 0 && full33(sm.stack.g[2]) && full33(sm.stack.g[1]);
-      for (int i = ci - 1; i >= (planar ? 2 : 1); --i)
+      if (fuse_z)
+      {
+        // (the same transform order: the inverse starts with Z too) the columns left
+        for (int li = tid; li < 17 * 17; li += kThreads)
+          dev::lift_line_strided<33, false, 33 * 33>(F + 2 * (li / 17) * 33 + 2 * (li % 17));
+        __syncthreads();
+      }
+      for (int i = fuse_z ? 1 : ci - 1; i >= (planar ? 2 : 1); --i)
       {
         dev::lift_sweep_regs<false>(F, N, sm.stack.g[i], sm.stack.axis[i]);
         __syncthreads();
       }
       ENC_PHASE(5)
-      if (planar)
-      {
-        constexpr int kPlanes = 4;  // 4 x 33 x 33 doubles: 34.8 KB, within the tables' space
-        double* T = reinterpret_cast<double*>(Xp);
-        for (int z0 = 0; z0 < 33; z0 += kPlanes)
-        {
-          const int nzc = 33 - z0 < kPlanes ? 33 - z0 : kPlanes;
-          const int n = nzc * 33 * 33;
-          const double* src = F + (size_t)z0 * 33 * 33;
-          for (int i = tid; i < n; i += kThreads)
-            T[i] = src[i];
-          __syncthreads();
-          // inverse Y (columns of each plane)
-          for (int li = tid; li < 33 * nzc; li += kThreads)
-            dev::lift_line_strided<33, false, 33>(T + (li / 33) * 33 * 33 + li % 33);
-          __syncthreads();
-          // inverse X (D = 33) then forward X of the one-level transform (Core/Wavelet.cpp:81)
-          for (int li = tid; li < 33 * nzc; li += kThreads)
-          {
-            double* row = T + li * 33;
-            double v[33];
-#pragma unroll
-            for (int k = 0; k < 33; ++k)
-              v[k] = row[k];
-            dev::lift_regs<false>(v, 33);
-            dev::lift_regs<true>(v, 33);
-#pragma unroll
-            for (int k = 0; k < 33; ++k)
-              row[k] = v[k];
-          }
-          __syncthreads();
-          // forward Y
-          for (int li = tid; li < 33 * nzc; li += kThreads)
-          {
-            double* col = T + (li / 33) * 33 * 33 + li % 33;
-            double v[33];
-#pragma unroll
-            for (int k = 0; k < 33; ++k)
-              v[k] = col[k * 33];
-            dev::lift_regs<true>(v, 33);
-#pragma unroll
-            for (int k = 0; k < 33; ++k)
-              col[k * 33] = v[k];
-          }
-          __syncthreads();
-          double* dst = F + (size_t)z0 * 33 * 33;
-          for (int i = tid; i < n; i += kThreads)
-            dst[i] = T[i];
-          __syncthreads();
-        }
-      }
+      if (planar && warp < nbufs)
+        for (int z = warp; z < 33; z += nbufs)
+          plane_middle(F + (size_t)z * kPlaneSamples, plane_buf, lane);
       // inverse X (D = 33) then forward X of the one-level transform (Core/Wavelet.cpp:81)
       for (int li = tid; !planar && li < 33 * N[2]; li += kThreads)
       {
