@@ -261,14 +261,14 @@ __device__ __forceinline__ void subband_grid(int is2d, int s, int from[3], int d
   }
 }
 
+// The largest of the lanes' non-negative values, by the order of their bits: two reductions in
+// hardware in place of five exchanges of doubles.
 __device__ __forceinline__ double warp_max(double v)
 {
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    double w = __shfl_xor_sync(0xffffffffu, v, o);
-    v = v < w ? w : v;
-  }
-  return v;
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned h = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
+  return __hiloint2double((int)h, (int)l);
 }
 
 // L2 prefetch of the field rows a level-0 brick will gather.
@@ -352,6 +352,8 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
   // significance chain and the plane lengths, lane-parallel over the planes.
   // The samples of the warp's next pair are loaded while the current pair is coded.
   const int npairs = (nb + 1) >> 1;
+  // the lane's places in a 4^3 block's coefficient order
+  const int p3a = qpad((int)sm.perm3[lane]), p3b = qpad((int)sm.perm3[lane + 32]);
   double cv[4];
   block_info cA, cB;
   auto load_pair = [&](int pr, double v[4], block_info& A, block_info& B) {
@@ -432,18 +434,18 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
       __syncwarp();
     }
     // shuffle to sequency order, negabinary (Core/Zfp.h:419-520)
-    auto permj = [&](int nd, int j) -> int {
-      return nd == 3 ? (int)sm.perm3[j] : (nd == 2 ? (int)sm.perm2[j & 15] : j);
+    auto permj = [&](int nd) -> int {  // (blocks of fewer than 64 values: the first 16 lanes)
+      return nd == 3 ? p3a : qpad(nd == 2 ? (int)sm.perm2[lane & 15] : lane);
     };
     unsigned long long uA0 = 0, uA1 = 0, uB0 = 0, uB1 = 0;
     if (lane < nvA)
-      uA0 = ((unsigned long long)qA[qpad(permj(ndA, lane))] + dev::kNegaMask) ^ dev::kNegaMask;
-    if (lane + 32 < nvA)
-      uA1 = ((unsigned long long)qA[qpad(permj(ndA, lane + 32))] + dev::kNegaMask) ^ dev::kNegaMask;
+      uA0 = ((unsigned long long)qA[permj(ndA)] + dev::kNegaMask) ^ dev::kNegaMask;
+    if (ndA == 3)
+      uA1 = ((unsigned long long)qA[p3b] + dev::kNegaMask) ^ dev::kNegaMask;
     if (lane < nvB)
-      uB0 = ((unsigned long long)qB[qpad(permj(ndB, lane))] + dev::kNegaMask) ^ dev::kNegaMask;
+      uB0 = ((unsigned long long)qB[permj(ndB)] + dev::kNegaMask) ^ dev::kNegaMask;
     if (lane + 32 < nvB)
-      uB1 = ((unsigned long long)qB[qpad(permj(ndB, lane + 32))] + dev::kNegaMask) ^ dev::kNegaMask;
+      uB1 = ((unsigned long long)qB[p3b] + dev::kNegaMask) ^ dev::kNegaMask;
     __syncwarp();
     int npA = dev::coded_planes(eA, fp.etol, fp.end_bp, fp.bpc);
     int npB = hasB ? dev::coded_planes(eB, fp.etol, fp.end_bp, fp.bpc) : 0;
@@ -498,19 +500,14 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
         if (k < npB)
           XB[k * kRowX] = xb;
         // inclusive maximum over planes <= k, i.e. over lanes >= lane
-        int ia = xa ? 64 - __clzll(xa) : 0, ib = xb ? 64 - __clzll(xb) : 0;
+        // (both blocks' in the halves of one word; a lane past the end gets its own value back)
+        unsigned iab = (unsigned)(64 - __clzll((long long)xa)) | ((unsigned)(64 - __clzll((long long)xb)) << 16);
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1)
-        {
-          const int ta = __shfl_down_sync(0xffffffffu, ia, o), tb = __shfl_down_sync(0xffffffffu, ib, o);
-          if (lane + o < 32)
-          {
-            ia = ia > ta ? ia : ta;
-            ib = ib > tb ? ib : tb;
-          }
-        }
-        int ea = __shfl_down_sync(0xffffffffu, ia, 1), eb = __shfl_down_sync(0xffffffffu, ib, 1);
-        ea = lane < 31 ? ea : 0;
-        eb = lane < 31 ? eb : 0;
+          iab = __vmaxu2(iab, __shfl_down_sync(0xffffffffu, iab, o));
+        unsigned eab = __shfl_down_sync(0xffffffffu, iab, 1);
+        eab = lane < 31 ? eab : 0u;
+        const int ea = (int)(eab & 0xffffu), eb = (int)(eab >> 16);
         const int nA_ = ea > carryA ? ea : carryA, nB_ = eb > carryB ? eb : carryB;
         if (k < npA)
         {
@@ -522,7 +519,8 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
           NIN[k * kRowNin + bB] = (uint8_t)nB_;
           OFF[k * kRowOff + bB] = (uint16_t)dev::plane_bits(xb, nB_, nvB);
         }
-        const int ta = __shfl_sync(0xffffffffu, ia, 0), tb = __shfl_sync(0xffffffffu, ib, 0);
+        const unsigned tab = __shfl_sync(0xffffffffu, iab, 0);
+        const int ta = (int)(tab & 0xffffu), tb = (int)(tab >> 16);
         carryA = carryA > ta ? carryA : ta;
         carryB = carryB > tb ? carryB : tb;
       }
