@@ -715,8 +715,7 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   cudaStream_t cs = split_out ? ctx->copies() : nullptr;
   stream_fence out_copies{ cs };  // band copies into the caller's buffer end before any return
   int* d_err = (int*)ctx->ws("dec.err", 16);  // [0] brick kernel, [1] plane kernels (bit flags)
-  uint64_t* d_geom = (uint64_t*)ctx->ws("dec.geom", sizeof(uint64_t) * 8 * kMaxBlocksPerSubband);
-  if (!d_err || !d_geom)
+  if (!d_err)
     return OutOfMemory;
   // the plane-table path's shared memory (float staging rows for a float32 output), and the
   // three-CTA build for an output level of many bricks with a float32 output
@@ -725,10 +724,15 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   // k_decode_level, as do several planes per key (other tables) and the coefficient mode.
   const bool by_lane = !r0.is2d && r0.bpc == 1 && !coeff_out;
   const size_t smem = by_lane ? sizeof(brick_smem<8>) : dec_smem_bytes(true, r0.f32);
-  cudaFuncSetAttribute(k_decode_bricks<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<8>));
-  cudaFuncSetAttribute(k_decode_bricks<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<16>));
-  cudaFuncSetAttribute(k_decode_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
-  cudaFuncSetAttribute(k_decode_level<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
+  if (!ctx->decode_kernels_set)
+  {
+    // once per context: the attributes stay with the device's functions
+    cudaFuncSetAttribute(k_decode_bricks<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<8>));
+    cudaFuncSetAttribute(k_decode_bricks<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<16>));
+    cudaFuncSetAttribute(k_decode_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
+    cudaFuncSetAttribute(k_decode_level<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
+    ctx->decode_kernels_set = true;
+  }
   int occ3 = 0;
   if (!by_lane && r0.f32 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_decode_level<3>, kThreads, smem) != cudaSuccess)
   {
@@ -840,8 +844,21 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
         std::stable_sort(hb.begin(), hb.end(),
                          [](const decode_brick& x, const decode_brick& y) { return x.dst_from[2] < y.dst_from[2]; });
       ++li;
-      decode_brick* d_bricks = (decode_brick*)ctx->ws("dec.bricks", sizeof(decode_brick) * (size_t)nbr);
-      decode_target* d_reqs = (decode_target*)ctx->ws("dec.reqs", sizeof(decode_target) * targets.size());
+      // the level's tables go up in one copy: the plane kernels' cursor and counter (zeros), the
+      // block walk, the requests, the bricks
+      const size_t gm_bytes = sizeof(uint64_t) * 8 * kMaxBlocksPerSubband;
+      const size_t tg_bytes = sizeof(decode_target) * targets.size();
+      const size_t hb_bytes = sizeof(decode_brick) * (size_t)nbr;
+      constexpr size_t o_geom = 256;
+      const size_t o_reqs = o_geom + gm_bytes;
+      const size_t o_bricks = (o_reqs + tg_bytes + 255) & ~(size_t)255;
+      uint8_t* d_tables = (uint8_t*)ctx->ws("dec.tables", o_bricks + hb_bytes);
+      if (!d_tables)
+        return OutOfMemory;
+      unsigned long long* d_pcur = (unsigned long long*)d_tables;
+      const uint64_t* d_geom = (const uint64_t*)(d_tables + o_geom);
+      const decode_target* d_reqs = (const decode_target*)(d_tables + o_reqs);
+      const decode_brick* d_bricks = (const decode_brick*)(d_tables + o_bricks);
       char kn[32];
       snprintf(kn, sizeof kn, "dec.keep%d", l);
       double* d_level = nstore ? (double*)ctx->ws(keep ? kn : (li % 2 ? "dec.levA" : "dec.levB"),
@@ -865,24 +882,20 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       const int cps = three ? 3 : 2;
       int grid = nbr < cps * ctx->num_sms ? nbr : cps * ctx->num_sms;
       double* d_slots = (double*)ctx->ws("dec.slots", (size_t)grid * (size_t)(by_lane ? kSlotBrick : NB) * 8);
-      if (!d_bricks || !d_reqs || (nstore && !d_level) || !d_slots)
+      if ((nstore && !d_level) || !d_slots)
         return OutOfMemory;
       // the level's tables through pinned staging of its own (copies stay asynchronous; the
       // call's final synchronisation comes before any reuse)
-      const size_t hb_bytes = sizeof(decode_brick) * (size_t)nbr;
-      const size_t tg_bytes = sizeof(decode_target) * targets.size();
-      const size_t gm_bytes = sizeof(uint64_t) * 8 * kMaxBlocksPerSubband;
       char pn[32];
       snprintf(pn, sizeof pn, "dec.hstage%d", l);
-      uint8_t* hs = (uint8_t*)ctx->pinned(pn, hb_bytes + tg_bytes + gm_bytes);
+      uint8_t* hs = (uint8_t*)ctx->pinned(pn, o_bricks + hb_bytes);
       if (!hs)
         return OutOfMemory;
-      memcpy(hs, hb.data(), hb_bytes);
-      memcpy(hs + hb_bytes, targets.data(), tg_bytes);
-      memcpy(hs + hb_bytes + tg_bytes, lw->geom, gm_bytes);
-      cudaMemcpyAsync(d_bricks, hs, hb_bytes, cudaMemcpyHostToDevice, st);
-      cudaMemcpyAsync(d_reqs, hs + hb_bytes, tg_bytes, cudaMemcpyHostToDevice, st);
-      cudaMemcpyAsync(d_geom, hs + hb_bytes + tg_bytes, gm_bytes, cudaMemcpyHostToDevice, st);
+      memset(hs, 0, o_geom);
+      memcpy(hs + o_geom, lw->geom, gm_bytes);
+      memcpy(hs + o_reqs, targets.data(), tg_bytes);
+      memcpy(hs + o_bricks, hb.data(), hb_bytes);
+      cudaMemcpyAsync(d_tables, hs, o_bricks + hb_bytes, cudaMemcpyHostToDevice, st);
       dec_args a;
       memset(&a, 0, sizeof a);
       a.level = l;
@@ -918,9 +931,8 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       // pass, whose count the kernel reads on the device
       const size_t nunits = (size_t)nbr * (size_t)r0.nsb;
       unsigned long long* d_uoff = (unsigned long long*)ctx->ws("dec.unitoff", nunits * 8);
-      unsigned long long* d_pcur = (unsigned long long*)ctx->ws("dec.pcursor", 16);
       int* d_wide = (int*)ctx->ws("dec.widelist", nunits * 4);
-      if (!d_uoff || !d_pcur || !d_wide)
+      if (!d_uoff || !d_wide)
         return OutOfMemory;
       unsigned long long cap = (unsigned long long)nunits * 16384ull + (16ull << 20);
       if (cap < min_cap)
@@ -959,7 +971,6 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
       pa.cap_bytes = cap;
       a.planes = d_planes;
       a.unit_off = d_uoff;
-      cudaMemsetAsync(d_pcur, 0, 16, st);
       cudaEvent_t t0 = ctx->ev(2 * nev), t1 = ctx->ev(2 * nev + 1);
       if (!t0 || !t1)
         return CudaError;

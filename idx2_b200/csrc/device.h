@@ -41,6 +41,7 @@ struct device_ctx
     return copy_out_stream;
   }
   long long launches = 0;  // kernels launched on this context so far
+  bool decode_kernels_set = false;  // the decode kernels' shared-memory limits are raised
   // batched encode: the launch shape chosen per batch signature (CTAs per SM + 10 * split kernel)
   std::map<std::string, int> tuned;
   std::shared_ptr<void> shard;       // a sharded encode between its two calls (api.cpp)
