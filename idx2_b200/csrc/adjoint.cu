@@ -40,12 +40,14 @@
 // the column pass. The order of the three CDF passes differs from the decode's Z, Y, X: they act
 // on different axes and commute, the results differ by rounding only.
 //
-// What bounds it: per brick 29 K cycles forward, of which the shared-memory pipe is busy half
+// What bounds it: per brick 26 K cycles forward, of which the shared-memory pipe is busy half
 // (some 10 accesses a sample) and the issue slots a third (38 K warp instructions), with the load
 // of a brick and the store of its grid not overlapped (one brick fills an SM). For 32 float fields
-// of 256^3 (gpu__time_duration, both levels) 1.86 ms forward and 2.18 ms adjoint; clusters of four
-// CTAs with every zfp pass and every sweep through shared memory took 3.09 and 2.69 ms, this
-// form over clusters of two CTAs, two clusters per SM pair, 2.09 and 2.26 ms.
+// of 256^3 (gpu__time_duration, both levels) 1.72 ms forward and 2.03 ms adjoint; with the Y and
+// the X sweep taken over all rows of the brick and a barrier between them, instead of a warp doing
+// both in its own plane (cdf_plane), 1.86 and 2.18 ms; that form over clusters of two CTAs, two
+// clusters per SM pair, 2.09 and 2.26 ms; clusters of four CTAs with every zfp pass and every
+// sweep through shared memory 3.09 and 2.69 ms.
 #include "codec_device.cuh"
 #include "device.h"
 #include "encoder.h"
@@ -390,38 +392,66 @@ __device__ __forceinline__ void face_x(T* S, int np, bool top, int tid, int nt)
   }
 }
 
-// CDF5/3 lines along y, with the de-normalisation before the lift (forward) or after the
-// transposed lift (adjoint).
+// One 33-sample line over the lanes of a warp: lane k holds samples 2k (k <= 16) and 2k + 1
+// (k <= 15); the operations of rilift33 / rilift33_adj, in their order.
 template <typename T, bool ADJ>
-__device__ __forceinline__ void cdf_y(const T* sw, T* S, int np, int z0, int tid, int nt)
+__device__ __forceinline__ void lift33_lanes(T& e, T& o, int lane)
 {
-  for (int L = tid; L < 33 * np; L += nt)
-  {
-    const int x = L % 33, p = L / 33;
-    const T w0 = sw[parity_index<false>(x, 0, z0 + p)], w1 = sw[parity_index<false>(x, 1, z0 + p)];
-    T* col = S + p * kLayer + x;
-    T v[33];
-#pragma unroll
-    for (int y = 0; y < 33; ++y)
-      v[y] = !ADJ ? col[y * kRow] * ((y & 1) ? w1 : w0) : col[y * kRow];
-    lift33<T, ADJ>(v);
-#pragma unroll
-    for (int y = 0; y < 33; ++y)
-      col[y * kRow] = ADJ ? v[y] * ((y & 1) ? w1 : w0) : v[y];
-  }
+  const T prev = __shfl_up_sync(0xffffffffu, o, 1);
+  constexpr T k = ADJ ? T(0.5) : T(-0.25);
+  if (ADJ && lane == 15)  // (rilift33_adj starts with the last odd sample)
+    e = axpb(o, k, e);
+  if (lane > 0)
+    e = axpb(prev, k, e);
+  if (lane < (ADJ ? 15 : 16))
+    e = axpb(o, k, e);
+  const T next = __shfl_down_sync(0xffffffffu, e, 1);
+  o = axpb(e + next, ADJ ? T(-0.25) : T(0.5), o);
 }
 
-// CDF5/3 lines along x, two samples an access (the 34th is padding).
+// The CDF5/3 sweeps inside plane z of the brick (at S), by a warp: along y with the
+// de-normalisation before it, then along x (forward), or along x, then along y with the
+// de-normalisation after it (adjoint). A lane per column or row, their 33rd over the lanes; rows two
+// samples an access (the 34th is padding).
 template <typename T, bool ADJ>
-__device__ __forceinline__ void cdf_x(T* S, int np, int tid, int nt)
+__device__ __forceinline__ void cdf_plane(const T* sw, T* S, int z, int lane)
 {
   struct alignas(2 * sizeof(T)) pair_t
   {
     T a, b;
   };
-  for (int L = tid; L < 33 * np; L += nt)
-  {
-    pair_t* row = reinterpret_cast<pair_t*>(S + (L / 33) * kLayer + (L % 33) * kRow);
+  const int l16 = lane < 16 ? lane : 16, l15 = lane < 15 ? lane : 15;
+  auto along_y = [&]() {
+    T e = S[2 * l16 * kRow + 32], o = S[(2 * l15 + 1) * kRow + 32];
+    T v[33];
+    const T w0 = sw[parity_index<false>(lane, 0, z)], w1 = sw[parity_index<false>(lane, 1, z)];
+    const T u0 = sw[parity_index<false>(32, 0, z)], u1 = sw[parity_index<false>(32, 1, z)];
+#pragma unroll
+    for (int y = 0; y < 33; ++y)
+      v[y] = !ADJ ? S[y * kRow + lane] * ((y & 1) ? w1 : w0) : S[y * kRow + lane];
+    if (!ADJ)
+    {
+      e *= u0;
+      o *= u1;
+    }
+    lift33_lanes<T, ADJ>(e, o, lane);
+    lift33<T, ADJ>(v);
+    if (ADJ)
+    {
+      e *= u0;
+      o *= u1;
+    }
+#pragma unroll
+    for (int y = 0; y < 33; ++y)
+      S[y * kRow + lane] = ADJ ? v[y] * ((y & 1) ? w1 : w0) : v[y];
+    if (lane < 17)
+      S[2 * lane * kRow + 32] = e;
+    if (lane < 16)
+      S[(2 * lane + 1) * kRow + 32] = o;
+  };
+  auto along_x = [&]() {
+    pair_t* row = reinterpret_cast<pair_t*>(S + lane * kRow);
+    pair_t last = reinterpret_cast<pair_t*>(S + 32 * kRow)[l16];
     T v[33];
 #pragma unroll
     for (int x = 0; x < 17; ++x)
@@ -431,10 +461,25 @@ __device__ __forceinline__ void cdf_x(T* S, int np, int tid, int nt)
       if (x < 16)
         v[2 * x + 1] = r.b;
     }
+    lift33_lanes<T, ADJ>(last.a, last.b, lane);
     lift33<T, ADJ>(v);
 #pragma unroll
     for (int x = 0; x < 17; ++x)
       row[x] = pair_t{ v[2 * x], x < 16 ? v[2 * x + 1] : T(0) };
+    if (lane < 17)
+      reinterpret_cast<pair_t*>(S + 32 * kRow)[lane] = last;
+  };
+  if constexpr (!ADJ)
+  {
+    along_y();
+    __syncwarp();
+    along_x();
+  }
+  else
+  {
+    along_x();
+    __syncwarp();
+    along_y();
   }
 }
 
@@ -539,9 +584,8 @@ __global__ void __launch_bounds__(syn3<T>::threads, 1) k_synth3(const syn_args<T
       __syncthreads();
       face_x<T, false>(S, np, top, tid, NT);
       __syncthreads();
-      cdf_y<T, false>(sw, S, np, z0, tid, NT);
-      __syncthreads();
-      cdf_x<T, false>(S, np, tid, NT);
+      for (int p = warp; p < np; p += NW)
+        cdf_plane<T, false>(sw, S + p * kLayer, z0 + p, lane);
       cluster_sync<CS>();
       // Z pass over the brick: this CTA's share of the columns (the grid has those below 32)
       const int side = a.finest ? 32 : 33;
@@ -641,9 +685,8 @@ __global__ void __launch_bounds__(syn3<T>::threads, 1) k_synth3(const syn_args<T
           prefetch_l2(g + nx.valid[0] - 1);
         }
       }
-      cdf_x<T, true>(S, np, tid, NT);
-      __syncthreads();
-      cdf_y<T, true>(sw, S, np, z0, tid, NT);
+      for (int p = warp; p < np; p += NW)
+        cdf_plane<T, true>(sw, S + p * kLayer, z0 + p, lane);
       __syncthreads();
       // transposed zfp: x, y, z; the low band over the uncoded blocks goes to the parent (and
       // nowhere else)
