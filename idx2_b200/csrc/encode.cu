@@ -1367,6 +1367,8 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
       const int nf = sm.stack.n, cf = sm.stack.coarse;
       // A column with x or y odd holds no sample of the lattice: its forward Z sweep is followed by
       // the inverse one at once (one read and one write of it less; 38.1 -> 37.3 ms at 1024^3).
+      // The others' even samples go to the lattice in shared memory from the registers, and come
+      // back from there into the inverse (two passes over them less; 33.3 -> 32.3 ms).
       const bool fuse_z = by_plane && cf == 3 && level_one(sm.stack.g[2]);
       if (fuse_z)
       {
@@ -1379,11 +1381,17 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
             v[k] = col[k * 33 * 33];
           v[32] = 0.0;
           dev::lift_regs<true>(v, 32);
-          if (((li % 33) | (li / 33)) & 1)
+          const int x = li % 33, y = li / 33;
+          const bool on_lattice = !((x | y) & 1);
+          if (!on_lattice)
             dev::lift_regs<false>(v, 33);
+          double* lat = S + (y >> 1) * 17 + (x >> 1);
 #pragma unroll
           for (int k = 0; k < 33; ++k)
-            col[k * 33 * 33] = v[k];
+            if (on_lattice && !(k & 1))
+              lat[(k >> 1) * 289] = v[k];
+            else
+              col[k * 33 * 33] = v[k];
         }
         __syncthreads();
       }
@@ -1397,12 +1405,15 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
         }
       }
       ENC_PHASE(2)
-      for (int i = tid; i < nsub; i += kThreads)
+      if (!fuse_z)
       {
-        const int x = i % 17, y = (i / 17) % 17, z = i / 289;
-        S[i] = F[(2 * z * 33 + 2 * y) * 33 + 2 * x];
+        for (int i = tid; i < nsub; i += kThreads)
+        {
+          const int x = i % 17, y = (i / 17) % 17, z = i / 289;
+          S[i] = F[(2 * z * 33 + 2 * y) * 33 + 2 * x];
+        }
+        __syncthreads();
       }
-      __syncthreads();
       const bool usual = sm.usual_lattice != 0;  // (then the inverse's stack is the usual one too)
       if (usual)
       {
@@ -1437,12 +1448,15 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
         dev::lift_sweep(S, NS, dev::half_grid(sm.stack.g[i]), NS, sm.stack.axis[i], false);
         __syncthreads();
       }
-      for (int i = tid; i < nsub; i += kThreads)
+      if (!fuse_z)
       {
-        const int x = i % 17, y = (i / 17) % 17, z = i / 289;
-        F[(2 * z * 33 + 2 * y) * 33 + 2 * x] = S[i];
+        for (int i = tid; i < nsub; i += kThreads)
+        {
+          const int x = i % 17, y = (i / 17) % 17, z = i / 289;
+          F[(2 * z * 33 + 2 * y) * 33 + 2 * x] = S[i];
+        }
+        __syncthreads();
       }
-      __syncthreads();
       ENC_PHASE(4)
       // With the first level's sweeps in Z, Y, X order on the whole 33^3 brick (the usual
       // transform order), the sweeps that stay inside z-planes -- the inverse Y, the inverse
@@ -1459,7 +1473,17 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
       {
         // (the same transform order: the inverse starts with Z too) the columns left
         for (int li = tid; li < 17 * 17; li += kThreads)
-          dev::lift_line_strided<33, false, 33 * 33>(F + 2 * (li / 17) * 33 + 2 * (li % 17));
+        {
+          double* col = F + 2 * (li / 17) * 33 + 2 * (li % 17);
+          double v[33];
+#pragma unroll
+          for (int k = 0; k < 33; ++k)
+            v[k] = k & 1 ? col[k * 33 * 33] : S[(k >> 1) * 289 + li];
+          dev::lift_regs<false>(v, 33);
+#pragma unroll
+          for (int k = 0; k < 33; ++k)
+            col[k * 33 * 33] = v[k];
+        }
         __syncthreads();
       }
       for (int i = fuse_z ? 1 : ci - 1; i >= (planar ? 2 : 1); --i)
