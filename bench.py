@@ -51,16 +51,16 @@ LEVELS = 3
 TOL = 1e-3
 METRIC = "encode+decode GB/s (raw field bytes) at 1e-3 tol"
 # DRAM bytes (read + write) of one level-0 k_encode_level launch per brick, from an ncu capture
-# of the grf512 workload (the three-CTA build, 444 CTAs, 4,096 bricks: 5.277 GB read + 4.294 GB
+# of the grf512 workload (444 CTAs, three per SM, 4,096 bricks: 3.613 GB read + 2.420 GB
 # written; the CTAs' FP64 brick slots, 122 MB, no longer fit in L2 beside the streams); the
 # traffic of a launch grows with its bricks (every brick makes the same slot sweeps on the same
 # grid), so a full launch's traffic is this figure times its bricks.
-ENC_L0_TRAFFIC_PER_BRICK = (5.277031e9 + 4.294031e9) / 4096
+ENC_L0_TRAFFIC_PER_BRICK = (3.612898e9 + 2.420102e9) / 4096
 # FP64 operations of one level-0 k_encode_level launch per brick, from the same kind of ncu
-# capture (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum: 2,872,791,040 adds,
-# 1,577,402,368 multiplies, no fused multiply-adds over 4,096 bricks); every brick runs the same
+# capture (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum: 2,918,006,784 adds,
+# 1,605,386,240 multiplies, no fused multiply-adds over 4,096 bricks); every brick runs the same
 # lifting sweeps, so a launch's count is this figure times its bricks.
-ENC_L0_FP64_OPS_PER_BRICK = (2872791040 + 1577402368) / 4096
+ENC_L0_FP64_OPS_PER_BRICK = (2918006784 + 1605386240) / 4096
 
 
 def fp64_peak(dev):
@@ -650,7 +650,7 @@ def ours(args, rank, world, local_rank):
                              "ops_per_brick": ENC_L0_FP64_OPS_PER_BRICK,
                              "ops_source": "ncu smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum of "
                                            "the level-0 launch at 512^3 (4,096 bricks), scaled by bricks"}
-    line["roofline_decode"] = {"bound": "hbm", "kernel": "k_decode_planes + k_decode_level (all levels)",
+    line["roofline_decode"] = {"bound": "hbm", "kernel": "k_decode_planes_ring + k_decode_bricks (all levels)",
                                "achieved": dec_bytes / (dec_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                                "frac": dec_bytes / (dec_ms * 1e-3) / 1e9 / peak, "algorithmic_bytes": dec_bytes}
     _lib.lib().idx2g_ctx_destroy(h)

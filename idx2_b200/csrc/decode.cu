@@ -1,6 +1,10 @@
 // Decode kernels for sm_100a (Core/idx2Decode.cpp:86-320, :431-442).
 //
-// One persistent CTA per brick slot. For every brick of a level:
+// Per level: the bit planes of every (brick, subband) unit into plane tables
+// (k_decode_planes_ring, k_decode_planes: decode_kernel.cuh), then the bricks. 3D bricks of one
+// plane per key: k_decode_bricks (decode_bricks.cuh). Others, the coefficient mode, and the
+// allocation-free decode (which takes the planes in the same kernel): k_decode_level, one
+// persistent CTA per brick slot, for every brick of a level:
 //   1  zero the FP64 brick, copy the parent's reconstructed low band into it,
 //   2  per decoded subband: read the block exponents, then decode the bit planes as
 //      a wavefront: thread j owns bit-plane channel (kmax - j) and its bit cursor;
@@ -717,8 +721,8 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   int* d_err = (int*)ctx->ws("dec.err", 16);  // [0] brick kernel, [1] plane kernels (bit flags)
   if (!d_err)
     return OutOfMemory;
-  // the plane-table path's shared memory (float staging rows for a float32 output), and the
-  // three-CTA build for an output level of many bricks with a float32 output
+  // k_decode_level's shared memory on plane tables (float staging rows for a float32 output), and
+  // its three-CTA build for an output level of many bricks with a float32 output
   // 3D bricks of one plane per key: k_decode_bricks (its header has both sides' times). Its
   // registers hold one 4^3 block per lane, so 2D bricks, whose blocks are 4 x 4, keep
   // k_decode_level, as do several planes per key (other tables) and the coefficient mode.

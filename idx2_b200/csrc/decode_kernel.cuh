@@ -470,8 +470,9 @@ __device__ __forceinline__ void plane_wavefront(const dec1_args& a, size_t fs, i
   }
 }
 
-// WIDE = false: every unit, those of up to 32 channels decoded at once (few registers, many
-// warps per SM), the others listed; WIDE = true: the listed units (up to kKeyWindow channels).
+// A pass over every unit decodes those of up to 32 channels at once (few registers, many warps per
+// SM: k_decode_planes_ring, or k_decode_planes<false, true> with several planes per key) and lists
+// the others; WIDE = true: the listed units (up to kKeyWindow channels).
 // A (brick, subband) unit of the plane kernel after its preparation: block tables filled,
 // channel window known, table allocated. run = 0: nothing to decode here (skipped, empty,
 // deferred to the second pass, or no room).

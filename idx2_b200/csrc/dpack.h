@@ -11,6 +11,8 @@
 // channel enters a chunk at the first brick of the range with bytes for it (at its place in
 // that brick's first-touch order of keys), which writes the data it held, and what it holds
 // at the end is written by FlushChunks in channel-key order. So:
+//   k_pack_exps writes the segments' raw exponents into the exponent buffer, first, so that the
+//     host compresses them (zstd) while the rest runs;
 //   the key pass (dpack.cu), over every event at once with a warp each: its region's key
 //     window and key-stream offsets, its segment's key range, then per key of the
 //     (level, subband, chunk) segment its brick count, first / last brick, byte and
@@ -18,11 +20,10 @@
 //     touch rank at which each key enters the chunk;
 //   the host orders the chunks by their flush stamps, assigns file offsets, builds the file
 //     tails and the statistics (no brick data touched);
-//   k_pack_write (a CTA per segment, a warp per chunk): exclusive scans over the segment's
+//   k_pack_write (2 to 8 CTAs per sub-range of a segment, a warp per key): exclusive scans over the
 //     bricks in encode order give each pair's place; the chunk header (varbyte NBricks, the
 //     first brick as a varbyte then unary gaps, varbyte sizes) and the pairs' channel bytes
-//     are scattered into the file images, and the raw exponents of the segment into the
-//     exponent buffer (compressed with zstd on the host).
+//     are scattered into the file images.
 // The files equal the host packer's (packer.cpp) byte for byte.
 #pragma once
 
