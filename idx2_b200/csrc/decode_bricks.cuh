@@ -12,9 +12,11 @@
 //    shuffles), and the inverse zfp runs on 64 registers of 32 bits: with at most 26 planes the
 //    low word of every 64-bit coefficient stays zero through the three passes (each pass needs
 //    two more bits, 26 + 6 = 32), so the high words alone give the 64-bit result exactly. Blocks
-//    of 27 to 44 planes are the exact sum of two such transforms (planes 0-25 and 26-43: the
-//    transform is linear where no halving loses a bit, which 64 - 44 - 6 > 0 spare bits ensure);
-//    only blocks of more planes take the warp-per-block 64-bit form.
+//    of 27 to 44 planes are the exact sum of two such transforms (planes 0-25 and 26-43): the
+//    transform is linear where no halving loses a bit, which 64 - 44 - 6 > 0 spare bits ensure,
+//    and where no halved value wraps around 64 bits, which the coder's blocks of finite samples
+//    are far from and which is checked (may_wrap). Blocks of more planes, and those that may wrap
+//    (a stream of another origin, or a damaged one), take the warp-per-block 64-bit form.
 //  * A warp's 32 blocks are the 8 blocks along z (4 of each z parity) of 4 tiles in a row along
 //    x, so the inverse CDF5/3 along z follows at once from shared memory, and the brick goes to
 //    its slot in L2 once, already swept along z.
@@ -215,6 +217,25 @@ __device__ __forceinline__ void inverse_zfp3(int32_t (&q)[64])
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     ilift4_w(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+}
+
+// Whether a halved value of the inverse transform of the 64-bit coefficients q * 2^32 + l, the l
+// (planes from kHighPlanes on) below 2^38, may come within 2^46 of the ends of the 64-bit range, so
+// that the sum of the two parts' transforms could differ from the transform of the sum. A pass
+// halves its w and y + w / 2; the passes before it give either at most 1.5^2 = 2.25 of any one
+// coefficient (the largest entry of ILift's matrix is 6/4), so with the sum of the |q| at most
+// 7 * 2^27 they stay below 0.985 * 2^31. Shifted down by 6 for the sum to fit, each rounded by less
+// than 1. (The coder's blocks hold |q| < 2^27 before its transform, which averages: the sum of all 64
+// coefficients is then at most 11.6 * 2^27, and 3 to 4 * 2^27 for white noise; one above the limit
+// only takes the slower form. The check costs 0.6% where every block has 27 to 44 planes: 256^3 float64
+// at 1e-7 1.048 -> 1.054 ms.)
+__device__ __forceinline__ bool may_wrap(const int32_t (&q)[64])
+{
+  uint32_t sum = 0;
+#pragma unroll
+  for (int j = 0; j < 64; ++j)
+    sum += (uint32_t)abs(q[j] >> 6);
+  return sum > (7u << 21) - 64u;
 }
 
 // What a lane knows of a block: its decoded planes (0: nothing to rebuild) and their words.
@@ -439,37 +460,41 @@ __device__ __forceinline__ void rebuild_tiles(const dec_args& a, brick_smem<W>& 
       for (int j = 0; j < 64; ++j)
         own[(j >> 4) * kTileRow + 4 * ((j & 3) + 4 * ((j >> 2) & 3))] = q[j];
     };
-    if (empty)
-      ;
-    else if (most <= kSplitPlanes)
+    bool wide = most > kSplitPlanes;
+    if (!empty && !wide)
     {
       int32_t q[64];
       if (most <= 16)
         block_words<16>(lb.row, 0, lb.np, 31, q);
       else
         block_words<32>(lb.row, 0, lb.np < kHighPlanes ? lb.np : kHighPlanes, 31, q);
-      inverse_zfp3(q);
-      put(q);
-      sm.scale[warp][lane] = lb.np ? __dmul_rn(dequant_scale(3, lb.emax), 4294967296.0) : 0.0;
       if (most > kHighPlanes)
+        wide = __any_sync(0xffffffffu, may_wrap(q));
+      if (!wide)
       {
-        // the planes past the 26th, added to the first part as 64-bit words
-        staged = false;
-        block_words<32>(lb.row, kHighPlanes, lb.np - kHighPlanes, 63 - kHighPlanes - kLowBase, q);
         inverse_zfp3(q);
-        const double scale = lb.np ? dequant_scale(3, lb.emax) : 0.0;
-        double* dst = F + (size_t)(8 * zb + hz) * kSlotPlane + slot_xy(8 * t + hx, 8 * yb + hy);
-#pragma unroll
-        for (int j = 0; j < 64; ++j)
+        put(q);
+        sm.scale[warp][lane] = lb.np ? __dmul_rn(dequant_scale(3, lb.emax), 4294967296.0) : 0.0;
+        if (most > kHighPlanes)
         {
-          const int32_t h = own[(j >> 4) * kTileRow + 4 * ((j & 3) + 4 * ((j >> 2) & 3))];
-          const long long u = (long long)(((unsigned long long)(uint32_t)h << 32) +
-                                          ((unsigned long long)(long long)q[j] << kLowBase));
-          dst[(j >> 4) * 2 * kSlotPlane + ((j >> 2) & 3) * 17 + (j & 3)] = __dmul_rn(scale, __ll2double_rn(u));
+          // the planes past the 26th, added to the first part as 64-bit words
+          staged = false;
+          block_words<32>(lb.row, kHighPlanes, lb.np - kHighPlanes, 63 - kHighPlanes - kLowBase, q);
+          inverse_zfp3(q);
+          const double scale = lb.np ? dequant_scale(3, lb.emax) : 0.0;
+          double* dst = F + (size_t)(8 * zb + hz) * kSlotPlane + slot_xy(8 * t + hx, 8 * yb + hy);
+#pragma unroll
+          for (int j = 0; j < 64; ++j)
+          {
+            const int32_t h = own[(j >> 4) * kTileRow + 4 * ((j & 3) + 4 * ((j >> 2) & 3))];
+            const long long u = (long long)(((unsigned long long)(uint32_t)h << 32) +
+                                            ((unsigned long long)(long long)q[j] << kLowBase));
+            dst[(j >> 4) * 2 * kSlotPlane + ((j >> 2) & 3) * 17 + (j & 3)] = __dmul_rn(scale, __ll2double_rn(u));
+          }
         }
       }
     }
-    else
+    if (wide)
     {
       staged = false;
       for (int r = 0; r < 32; ++r)
