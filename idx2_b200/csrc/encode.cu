@@ -1589,6 +1589,38 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
   ENC_PHASE_FLUSH
 }
 
+// Of a brick whose least or greatest sample is a zero: its first zero (z, then y, then x), sign
+// included, to out[0]. The value range of a field with zeros of both signs has the sign of the first
+// one in brick order, as the reference's sequential comparison leaves it (Core/Volume.h:1123); the
+// encode kernels' minima and maxima are of equal value, of whichever zero comes first in their own
+// orders. One CTA, and only for such fields: 32^3 samples from L2.
+__global__ void __launch_bounds__(256) k_first_zero(const enc_brick* bricks, const enc_field* fields, int bi,
+                                                    double* out)
+{
+  __shared__ int at;
+  const enc_brick& br = bricks[bi];
+  const enc_field& fp = fields[br.field];
+  const int vx = br.valid[0], vy = br.valid[1], n = vx * vy * br.valid[2];
+  const long long z0 = (long long)br.b3[2] * (fp.is2d ? 1 : 32), y0 = (long long)br.b3[1] * 32,
+                  x0 = (long long)br.b3[0] * 32;
+  auto sample = [&](int i) {
+    const long long src = ((z0 + i / (vx * vy)) * fp.fdims[1] + y0 + i / vx % vy) * fp.fdims[0] + x0 + i % vx;
+    return fp.field_f32 ? (double)((const float*)fp.field)[src] : ((const double*)fp.field)[src];
+  };
+  if (threadIdx.x == 0)
+    at = n;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += 256)
+    if (sample(i) == 0.0)
+    {
+      atomicMin(&at, i);
+      break;
+    }
+  __syncthreads();
+  if (threadIdx.x == 0 && at < n)
+    out[0] = sample(at);
+}
+
 namespace cg = cooperative_groups;
 #include "encode_split.cuh"
 
@@ -2340,6 +2372,30 @@ int batch_encoder::collect_level(int l, bool keep_device)
         bf.vmin = a0 < bf.vmin ? a0 : bf.vmin;
         bf.vmax = bf.vmax < a1 ? a1 : bf.vmax;
       }
+  }
+  // a zero that ends a field's range has the sign of the field's first zero (k_first_zero): that of
+  // the first brick whose own range ends in it
+  for (size_t fi = 0; l == 0 && nbr > 0 && fi < ll.fields.size(); ++fi)
+  {
+    batch_field& bf = J[(size_t)ll.field_job[fi]];
+    if (bf.vmin != 0 && bf.vmax != 0)
+      continue;
+    const std::vector<double>& ends = bf.vmin == 0 ? mn : mx;
+    const int j0 = ll.job_first[(size_t)ll.field_job[fi]];
+    const int jn = (int)bf.plan->levels[0].size();
+    const int bi = (int)(std::find(ends.begin() + j0, ends.begin() + j0 + jn, 0.0) - ends.begin());
+    if (bi == j0 + jn)
+      continue;
+    double zero = 0;
+    k_first_zero<<<1, 256, 0, st>>>(ll.args.bricks, ll.args.fields, bi, ll.d_bmin + bi);
+    ++ctx_->launches;
+    cudaMemcpyAsync(&zero, ll.d_bmin + bi, 8, cudaMemcpyDeviceToHost, st);
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+      return CudaError;
+    if (bf.vmin == 0)
+      bf.vmin = zero;
+    if (bf.vmax == 0)
+      bf.vmax = zero;
   }
   return NoError;
 }
