@@ -4,8 +4,10 @@
 // page faults of a fresh array included: 38 MB into a new numpy array took 8.2 ms, 4.6 GB/s. Here
 // up to 12 threads take pieces of 1 MB, each through a pinned piece of its own, so that the
 // faults, the host copies and the transfers of different pieces overlap (that copy: 1.7 ms, 16 host
-// cores). Copies of less than 4 MB, and those to or from pinned memory, stay one cudaMemcpyAsync:
-// threads would cost more than they save (12 of them start in some 0.2 ms).
+// cores). Copies of less than 4 MB stay one cudaMemcpyAsync, as threads would cost more than they save
+// (12 of them start in some 0.2 ms), and so do those to or from memory that CUDA knows: pinned, where
+// there is nothing to save, and managed memory or a device's, which cudaMemcpyAsync takes too and the
+// host copy may not reach.
 #pragma once
 
 #include "device.h"
@@ -24,13 +26,16 @@ constexpr size_t kHostCopyMin = (size_t)4 << 20;
 constexpr unsigned kHostCopyThreads = 12;
 constexpr size_t kHostCopyEvents = 96;  // events of the context's pool from here on (no other user's)
 
-inline bool is_pinned(const void* p)
+inline bool is_memory(const void* p, cudaMemoryType type)
 {
   cudaPointerAttributes pa;
-  const bool pinned = cudaPointerGetAttributes(&pa, p) == cudaSuccess && pa.type == cudaMemoryTypeHost;
+  const bool is = cudaPointerGetAttributes(&pa, p) == cudaSuccess && pa.type == type;
   cudaGetLastError();
-  return pinned;
+  return is;
 }
+inline bool is_pinned(const void* p) { return is_memory(p, cudaMemoryTypeHost); }
+// memory that CUDA does not know; managed memory, or a device pointer given as a host one, is neither
+inline bool is_pageable(const void* p) { return is_memory(p, cudaMemoryTypeUnregistered); }
 
 // `bytes` from src to dst, one of them in device memory (to_host: src), in order after the work
 // of stream `st`. On return a copy to the host is done, or enqueued on `st` where it took the
@@ -43,7 +48,7 @@ inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, 
   if (nt > n)
     nt = (unsigned)n;
   uint8_t* slots = nullptr;
-  if (bytes >= kHostCopyMin && nt >= 2 && !is_pinned(to_host ? dst : src))
+  if (bytes >= kHostCopyMin && nt >= 2 && is_pageable(to_host ? dst : src))
     slots = (uint8_t*)ctx->pinned("host.slots", nt * kHostPiece);
   for (unsigned t = 0; slots && t < nt; ++t)
     if (!ctx->ev(kHostCopyEvents + t))

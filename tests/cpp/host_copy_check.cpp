@@ -1,0 +1,113 @@
+// Test driver: host_copy (host_copy.h) over a fake CUDA runtime. "Device memory" is ordinary memory
+// here; the fake counts the copies, and gives pointers the type that a case asks for. Runs the case
+// named on the command line, prints "ok" or the first failure; exit code 0 on success.
+#include "host_copy.h"
+
+#include <atomic>
+#include <cstdio>
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+using namespace idx2g;
+
+namespace
+{
+cudaMemoryType g_type = cudaMemoryTypeUnregistered;
+std::atomic<int> g_copies{ 0 };
+std::atomic<size_t> g_events{ 0 };
+} // namespace
+
+extern "C"
+{
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*)
+{
+  memset(a, 0, sizeof *a);
+  a->type = g_type;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t)
+{
+  ++g_copies;
+  memcpy(dst, src, n);
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e)
+{
+  *e = (cudaEvent_t)(++g_events);
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaMallocHost(void** p, size_t n)
+{
+  *p = malloc(n);
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p)
+{
+  free(p);
+  return cudaSuccess;
+}
+} // extern "C"
+
+namespace
+{
+
+int fail(const char* what, long long v)
+{
+  std::printf("FAIL %s %lld\n", what, v);
+  return 1;
+}
+
+// n bytes each way; the number of copies it took, or -1 where they do not arrive
+int copies_of(device_ctx* ctx, size_t n, bool to_host)
+{
+  std::vector<uint8_t> a(n), b(n, 0);
+  for (size_t i = 0; i < n; ++i)
+    a[i] = (uint8_t)(i * 31 + (i >> 8) + (i >> 16));
+  g_copies = 0;
+  if (host_copy(ctx, b.data(), a.data(), n, to_host, nullptr) != NoError || a != b)
+    return -1;
+  return g_copies;
+}
+
+// memory that CUDA knows (pinned, managed, a device's) stays one cudaMemcpyAsync, which takes any of
+// them; only memory that it does not know goes through the threads
+int registered()
+{
+  device_ctx ctx;
+  const bool threads = std::thread::hardware_concurrency() >= 2;
+  const size_t sizes[] = { 100, kHostCopyMin - 1, kHostCopyMin, kHostCopyMin + 3, 7 * kHostPiece + 12345 };
+  for (size_t n : sizes)
+    for (int to_host = 0; to_host < 2; ++to_host)
+    {
+      for (cudaMemoryType t : { cudaMemoryTypeHost, cudaMemoryTypeDevice, cudaMemoryTypeManaged })
+      {
+        g_type = t;
+        if (const int c = copies_of(&ctx, n, to_host != 0); c != 1)
+          return fail("registered: copies", c);
+      }
+      g_type = cudaMemoryTypeUnregistered;
+      const int want = n < kHostCopyMin || !threads ? 1 : (int)((n + kHostPiece - 1) / kHostPiece);
+      if (const int c = copies_of(&ctx, n, to_host != 0); c != want)
+        return fail("pageable: copies", c);
+    }
+  return 0;
+}
+
+} // namespace
+
+int main(int argc, char** argv)
+{
+  const std::string name = argc > 1 ? argv[1] : "";
+  int rc = 2;
+  if (name == "registered")
+    rc = registered();
+  if (rc == 0)
+    std::printf("ok\n");
+  return rc;
+}
