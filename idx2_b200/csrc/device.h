@@ -220,6 +220,20 @@ struct device_ctx
     }
     return evpool[i];
   }
+  // Events of the threads of a copy to or from pageable memory (host_copy.h), waited for by them
+  // alone: apart from the pool, whose users number its events each for themselves.
+  std::vector<cudaEvent_t> copy_events;
+  cudaEvent_t copy_ev(size_t i)
+  {
+    while (copy_events.size() <= i)
+    {
+      cudaEvent_t e = nullptr;
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+        return nullptr;
+      copy_events.push_back(e);
+    }
+    return copy_events[i];
+  }
   void release()
   {
     for (auto& kv : graphs)
@@ -236,6 +250,9 @@ struct device_ctx
     for (cudaEvent_t e : evpool)
       cudaEventDestroy(e);
     evpool.clear();
+    for (cudaEvent_t e : copy_events)
+      cudaEventDestroy(e);
+    copy_events.clear();
     for (auto& kv : bufs)
       if (kv.second.p)
         cudaFree(kv.second.p);

@@ -24,7 +24,6 @@ namespace idx2g
 constexpr size_t kHostPiece = (size_t)1 << 20;
 constexpr size_t kHostCopyMin = (size_t)4 << 20;
 constexpr unsigned kHostCopyThreads = 12;
-constexpr size_t kHostCopyEvents = 96;  // events of the context's pool from here on (no other user's)
 
 inline bool is_memory(const void* p, cudaMemoryType type)
 {
@@ -51,7 +50,7 @@ inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, 
   if (bytes >= kHostCopyMin && nt >= 2 && is_pageable(to_host ? dst : src))
     slots = (uint8_t*)ctx->pinned("host.slots", nt * kHostPiece);
   for (unsigned t = 0; slots && t < nt; ++t)
-    if (!ctx->ev(kHostCopyEvents + t))
+    if (!ctx->copy_ev(t))
       slots = nullptr;
   if (!slots)
   {
@@ -62,7 +61,7 @@ inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, 
   std::atomic<int> bad{ 0 };
   auto work = [&](unsigned t) {
     uint8_t* slot = slots + t * kHostPiece;
-    const cudaEvent_t ev = ctx->evpool[kHostCopyEvents + t];
+    const cudaEvent_t ev = ctx->copy_events[t];
     bool ok = cudaSetDevice(ctx->device) == cudaSuccess;
     for (size_t k; ok && (k = next.fetch_add(1)) < n;)
     {

@@ -16,6 +16,8 @@ namespace
 cudaMemoryType g_type = cudaMemoryTypeUnregistered;
 std::atomic<int> g_copies{ 0 };
 std::atomic<size_t> g_events{ 0 };
+std::mutex g_lock;
+std::vector<cudaEvent_t> g_recorded;
 } // namespace
 
 extern "C"
@@ -37,7 +39,13 @@ cudaError_t cudaEventCreate(cudaEvent_t* e)
   *e = (cudaEvent_t)(++g_events);
   return cudaSuccess;
 }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t)
+{
+  const std::lock_guard<std::mutex> lock(g_lock);
+  g_recorded.push_back(e);
+  return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
@@ -99,6 +107,25 @@ int registered()
   return 0;
 }
 
+// the threads' events are no event of the pool that encodes, decodes and the packer number for
+// themselves (the packer one for every 32 MB of an image, without a bound)
+int events()
+{
+  device_ctx ctx;
+  std::vector<cudaEvent_t> pool;
+  for (size_t i = 0; i < 400; ++i)
+    pool.push_back(ctx.ev(i));
+  g_type = cudaMemoryTypeUnregistered;
+  g_recorded.clear();
+  if (copies_of(&ctx, 5 * kHostPiece, true) < 1)
+    return fail("events: copies", -1);
+  for (cudaEvent_t e : g_recorded)
+    for (size_t i = 0; i < pool.size(); ++i)
+      if (e == pool[i])
+        return fail("events: of the pool", (long long)i);
+  return 0;
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -107,6 +134,8 @@ int main(int argc, char** argv)
   int rc = 2;
   if (name == "registered")
     rc = registered();
+  else if (name == "events")
+    rc = events();
   if (rc == 0)
     std::printf("ok\n");
   return rc;
