@@ -38,7 +38,8 @@ inline bool is_pageable(const void* p) { return is_memory(p, cudaMemoryTypeUnreg
 
 // `bytes` from src to dst, one of them in device memory (to_host: src), in order after the work
 // of stream `st`. On return a copy to the host is done, or enqueued on `st` where it took the
-// plain form; a pageable source is no longer read. Returns an error code.
+// plain form; a pageable source is no longer read. Returns an error code; then nothing is in flight
+// on `st` any more, neither the copies of the threads nor earlier ones of the caller's.
 inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, bool to_host, cudaStream_t st)
 {
   const size_t n = (bytes + kHostPiece - 1) / kHostPiece;
@@ -54,8 +55,10 @@ inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, 
       slots = nullptr;
   if (!slots)
   {
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
-    return e == cudaSuccess ? NoError : CudaError;
+    if (cudaMemcpyAsync(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st) == cudaSuccess)
+      return NoError;
+    cudaStreamSynchronize(st);
+    return CudaError;
   }
   std::atomic<size_t> next{ 0 };
   std::atomic<int> bad{ 0 };
@@ -91,7 +94,10 @@ inline int host_copy(device_ctx* ctx, void* dst, const void* src, size_t bytes, 
   work(0);
   for (auto& t : th)
     t.join();
-  return bad ? CudaError : NoError;
+  if (!bad)
+    return NoError;
+  cudaStreamSynchronize(st);
+  return CudaError;
 }
 
 } // namespace idx2g

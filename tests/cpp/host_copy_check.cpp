@@ -18,6 +18,8 @@ std::atomic<int> g_copies{ 0 };
 std::atomic<size_t> g_events{ 0 };
 std::mutex g_lock;
 std::vector<cudaEvent_t> g_recorded;
+int g_fail_copy = -1, g_fail_record = -1;  // the call, counted from 0, that fails
+bool g_in_flight = false;                  // copies since the last wait for the stream
 } // namespace
 
 extern "C"
@@ -30,7 +32,13 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*)
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t)
 {
-  ++g_copies;
+  {
+    const std::lock_guard<std::mutex> lock(g_lock);
+    if (g_copies == g_fail_copy)
+      return cudaErrorInvalidValue;
+    ++g_copies;
+    g_in_flight = true;
+  }
   memcpy(dst, src, n);
   return cudaSuccess;
 }
@@ -43,11 +51,18 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEven
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t)
 {
   const std::lock_guard<std::mutex> lock(g_lock);
+  if ((int)g_recorded.size() == g_fail_record)
+    return cudaErrorInvalidResourceHandle;
   g_recorded.push_back(e);
   return cudaSuccess;
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t)
+{
+  const std::lock_guard<std::mutex> lock(g_lock);
+  g_in_flight = false;
+  return cudaSuccess;
+}
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n)
@@ -126,6 +141,33 @@ int events()
   return 0;
 }
 
+// a copy that fails, in either form and at any call, says so, and leaves none in flight on the stream:
+// the caller returns with the error, and its buffers may go
+int failures()
+{
+  device_ctx ctx;
+  std::vector<uint8_t> a(6 * kHostPiece), b(6 * kHostPiece);
+  g_type = cudaMemoryTypeUnregistered;
+  for (size_t n : { (size_t)1000, b.size() })
+    for (int to_host = 0; to_host < 2; ++to_host)
+      for (int k = 0; k < 12; ++k)
+      {
+        g_copies = 0;
+        g_recorded.clear();
+        g_fail_copy = k % 2 ? -1 : k / 2;
+        g_fail_record = k % 2 ? k / 2 : -1;
+        if (n < kHostCopyMin && k)
+          continue;
+        g_in_flight = true;  // an earlier copy of the caller's
+        if (host_copy(&ctx, b.data(), a.data(), n, to_host != 0, nullptr) == NoError &&
+            std::thread::hardware_concurrency() >= 2)
+          return fail("failures: not said", k);
+        if (g_in_flight && std::thread::hardware_concurrency() >= 2)
+          return fail("failures: in flight", k);
+      }
+  return 0;
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -136,6 +178,8 @@ int main(int argc, char** argv)
     rc = registered();
   else if (name == "events")
     rc = events();
+  else if (name == "failures")
+    rc = failures();
   if (rc == 0)
     std::printf("ok\n");
   return rc;

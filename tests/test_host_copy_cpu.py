@@ -22,7 +22,7 @@ def check():
     return exe
 
 
-@pytest.mark.parametrize("case", ["registered", "events"])
+@pytest.mark.parametrize("case", ["registered", "events", "failures"])
 def test_host_copy(check, case):
     r = subprocess.run([check, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
