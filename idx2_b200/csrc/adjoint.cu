@@ -956,6 +956,11 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
   cudaStream_t st = ctx->stream;
   const long long gcount = (long long)f.dims.x * f.dims.y * f.dims.z;
   T* prev = nullptr;  // forward: kept bricks of the coarser level; adjoint: this level's gradient bricks
+  // an error return waits for the levels launched so far: they read and write the caller's arrays
+  auto fail = [st](int e) {
+    cudaStreamSynchronize(st);
+    return e;
+  };
   for (int step = 0; step < L; ++step)
   {
     const int l = adjoint ? step : L - 1 - step;
@@ -988,7 +993,7 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
       {
         a.bricks_out = (T*)ctx->ws(nm, (size_t)a.nbricks * (size_t)NB * sizeof(T));
         if (!a.bricks_out)
-          return OutOfMemory;
+          return fail(OutOfMemory);
       }
     }
     else
@@ -1000,23 +1005,23 @@ int run_synth(device_ctx* ctx, const dataset_format& f, int nbatch, const void* 
         const size_t pn = (size_t)a.npb[0] * (size_t)a.npb[1] * (size_t)a.npb[2] * (size_t)nbatch * (size_t)NB;
         a.pgrad = (T*)ctx->ws(nm, pn * sizeof(T));
         if (!a.pgrad)
-          return OutOfMemory;
+          return fail(OutOfMemory);
         cudaMemsetAsync(a.pgrad, 0, pn * sizeof(T), st);
       }
     }
     // the levels follow one another on the stream; the host waits once, after the last
     cudaEvent_t t0 = ctx->ev((size_t)(2 * step)), t1 = ctx->ev((size_t)(2 * step + 1));
     if (!t0 || !t1)
-      return CudaError;
+      return fail(CudaError);
     cudaEventRecord(t0, st);
     const int e = f.is2d() ? launch_synth<T, true>(ctx, a, adjoint, st) : launch_synth<T, false>(ctx, a, adjoint, st);
     cudaEventRecord(t1, st);
     if (e)
-      return e;
+      return fail(e);
     prev = adjoint ? a.pgrad : a.bricks_out;
     ++ctx->launches;
     if (cudaGetLastError() != cudaSuccess)
-      return CudaError;
+      return fail(CudaError);
   }
   if (cudaStreamSynchronize(st) != cudaSuccess)
     return CudaError;
