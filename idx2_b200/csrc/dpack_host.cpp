@@ -2,13 +2,13 @@
 // between the host stages of dpack_plan.cpp, and the encode path that uses them.
 #include "dpack_device.h"
 
+#include "parallel.h"
 #include "trace.h"
 
 #include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <fcntl.h>
-#include <system_error>
 #include <thread>
 #include <unistd.h>
 
@@ -156,29 +156,11 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
     return CudaError;
   std::vector<std::vector<uint8_t>> frames;
   int frames_err = NoError;
-  std::thread compress;
-  struct compress_joiner
-  {
-    std::thread& t;
-    ~compress_joiner()
-    {
-      if (t.joinable())
-        t.join();
-    }
-  } join_compress{ compress };
-  auto make_frames = [&frames, &frames_err, &P, h_exps, ex, dev = ctx->device]() {
+  side_task compress([&frames, &frames_err, &P, h_exps, ex, dev = ctx->device] {
     frames_err = cudaSetDevice(dev) == cudaSuccess && cudaEventSynchronize(ex) == cudaSuccess
                    ? dpack_compress(P, h_exps, &frames)
                    : CudaError;
-  };
-  try
-  {
-    compress = std::thread(make_frames);
-  }
-  catch (const std::system_error&)
-  {
-    // no thread to be had: compressed below, after the packing
-  }
+  });
   // the key pass (a warp per event, a CTA per sub-range for the totals, a CTA per segment for
   // the ranks); k_pack_write: a warp per key of a sub-range
   const int grid = nseg < 4 * ctx->num_sms ? nseg : 4 * ctx->num_sms;
@@ -239,10 +221,7 @@ int device_pack(device_ctx* ctx, const dataset_format& f, const std::shared_ptr<
   out->image = h_img;
   if (on_image)
     on_image(L, h_img, out->ready);  // e.g. the chunk sections written while the rest is made
-  if (compress.joinable())
-    compress.join();
-  else
-    make_frames();
+  compress.wait();
   if (frames_err)
     return frames_err;
   tt.lap("dpack.write");

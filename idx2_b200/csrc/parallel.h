@@ -4,7 +4,11 @@
 
 #include <atomic>
 #include <cstddef>
+#include <exception>
+#include <functional>
+#include <system_error>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace idx2g
@@ -45,5 +49,57 @@ void parallel_ranges(size_t n, F&& f)
     f(i0, i0 + step < n ? i0 + step : n);
   });
 }
+
+// A function that runs on a thread of its own beside its maker, or inside wait() where no thread
+// is to be had. wait() returns once it has run, and throws what it threw, which must not leave the
+// thread (the process would end there); a task destroyed without wait() is joined.
+class side_task
+{
+public:
+  explicit side_task(std::function<void()> f) : f_(std::move(f))
+  {
+    try
+    {
+      thread_ = std::thread([this] { run(); });
+    }
+    catch (const std::system_error&)
+    {
+      // no thread: wait() runs it
+    }
+  }
+  ~side_task()
+  {
+    if (thread_.joinable())
+      thread_.join();
+  }
+  side_task(const side_task&) = delete;
+  side_task& operator=(const side_task&) = delete;
+  void wait()
+  {
+    if (thread_.joinable())
+      thread_.join();
+    else if (f_)
+      run();
+    if (error_)
+      std::rethrow_exception(std::exchange(error_, nullptr));
+  }
+
+private:
+  void run()
+  {
+    try
+    {
+      f_();
+    }
+    catch (...)
+    {
+      error_ = std::current_exception();
+    }
+    f_ = nullptr;
+  }
+  std::function<void()> f_;
+  std::exception_ptr error_;
+  std::thread thread_;
+};
 
 } // namespace idx2g
