@@ -721,22 +721,26 @@ int decode_device::decode_batch(device_ctx* ctx, const std::vector<const decode_
   int* d_err = (int*)ctx->ws("dec.err", 16);  // [0] brick kernel, [1] plane kernels (bit flags)
   if (!d_err)
     return OutOfMemory;
-  // k_decode_level's shared memory on plane tables (float staging rows for a float32 output), and
-  // its three-CTA build for an output level of many bricks with a float32 output
   // 3D bricks of one plane per key: k_decode_bricks (its header has both sides' times). Its
   // registers hold one 4^3 block per lane, so 2D bricks, whose blocks are 4 x 4, keep
   // k_decode_level, as do several planes per key (other tables) and the coefficient mode.
   const bool by_lane = !r0.is2d && r0.bpc == 1 && !coeff_out;
   const size_t smem = by_lane ? sizeof(brick_smem<8>) : dec_smem_bytes(true, r0.f32);
-  if (!ctx->decode_kernels_set)
+  // (once per context: the limits stay with the device's functions)
+  if (!raise_smem_limits(&ctx->decode_kernels_set,
+                         { { (const void*)k_decode_bricks<8>, sizeof(brick_smem<8>) },
+                           { (const void*)k_decode_bricks<16>, sizeof(brick_smem<16>) },
+                           { (const void*)k_decode_level<2>, sizeof(dec_smem) },
+                           { (const void*)k_decode_level<3>, sizeof(dec_smem) } },
+                         [](const void* k, size_t n) {
+                           return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n) ==
+                                  cudaSuccess;
+                         }))
   {
-    // once per context: the attributes stay with the device's functions
-    cudaFuncSetAttribute(k_decode_bricks<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<8>));
-    cudaFuncSetAttribute(k_decode_bricks<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(brick_smem<16>));
-    cudaFuncSetAttribute(k_decode_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
-    cudaFuncSetAttribute(k_decode_level<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dec_smem));
-    ctx->decode_kernels_set = true;
+    cudaGetLastError();
+    return CudaError;
   }
+  // k_decode_level's three-CTA build for an output level of many bricks with a float32 output
   int occ3 = 0;
   if (!by_lane && r0.f32 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_decode_level<3>, kThreads, smem) != cudaSuccess)
   {

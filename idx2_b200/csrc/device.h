@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstdlib>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <string>
@@ -13,6 +14,26 @@
 
 namespace idx2g
 {
+
+struct kernel_smem
+{
+  const void* kernel;
+  size_t bytes;
+};
+
+// Raises the kernels' shared-memory limits with set(kernel, bytes), unless *done says that they are
+// raised; *done is set once all of them are, so that a call after a failed one tries again.
+template <typename Set>
+bool raise_smem_limits(bool* done, std::initializer_list<kernel_smem> kernels, Set set)
+{
+  if (*done)
+    return true;
+  for (const kernel_smem& k : kernels)
+    if (!set(k.kernel, k.bytes))
+      return false;
+  *done = true;
+  return true;
+}
 
 // One context per thread; all work is ordered on `stream`. The context owns a
 // grow-only workspace of named device buffers reused across calls, so repeated
