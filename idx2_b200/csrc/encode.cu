@@ -171,8 +171,8 @@ using enc_smem = enc_smem_t<kThreads>;
 // as the tables' space holds (6 of the 8 warps for float32 data, all of them for float64; a third
 // CTA per SM is worth more than the other two).
 constexpr int kPlaneSamples = 33 * 33;
-constexpr int kPlaneBufs = 6;
-static_assert(kWarps >= 8, "plane buffers belong to warps");
+constexpr __host__ __device__ int plane_bufs(int planes) { return planes == 32 ? 6 : 8; }
+static_assert(kWarps >= plane_bufs(32) && kWarps >= plane_bufs(64), "plane buffers belong to warps");
 
 inline size_t enc_smem_bytes(int planes)
 {
@@ -183,7 +183,7 @@ inline size_t enc_smem_bytes(int planes)
   const size_t band = (size_t)kGz * 32 * 32 * (planes == 32 ? 4 : 8) + (size_t)kGz * 33 * 33 * 8;
   size_t space = tables > lattice ? tables : lattice;
   space = space > band ? space : band;
-  const size_t bufs = (size_t)kPlaneBufs * kPlaneSamples * 8;
+  const size_t bufs = (size_t)plane_bufs(planes) * kPlaneSamples * 8;
   space = space > bufs ? space : bufs;
   return ((sizeof(enc_smem) + 127) & ~(size_t)127) + space;
 }
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(kThreads, CPS) k_encode_level(const enc_args a
     const bool by_plane = !fp.is2d && br.valid[0] == 32 && br.valid[1] == 32 && br.valid[2] == 32 &&
                           sm.stack.coarse >= 3 && sm.stack.axis[0] == 0 && sm.stack.axis[1] == 1 &&
                           sm.stack.axis[2] == 2 && level_one(sm.stack.g[0]) && level_one(sm.stack.g[1]);
-    const int nbufs = P == 32 ? kPlaneBufs : 8;
+    const int nbufs = plane_bufs(P);
     double* const plane_buf = reinterpret_cast<double*>(Xp) + (size_t)warp * kPlaneSamples;
     ENC_PHASE_START
     // ---------------- A: gather ----------------
