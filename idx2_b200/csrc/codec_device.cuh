@@ -558,13 +558,13 @@ __device__ __forceinline__ void warp_inv_zfp(long long* q, int nd, int lane)
 constexpr unsigned long long kNegaMask = 0xaaaaaaaaaaaaaaaaull;
 
 // Coefficient order by total sequency (Core/Zfp.h:419 Perm3, :498 Perm2), as flat
-// indices x + 4y + 16z into the block.
-static __constant__ uint8_t kPerm3d[64] = {
+// indices x + 4y + 16z into the block (constexpr: register numbers in unrolled loops).
+static __constant__ constexpr uint8_t kPerm3d[64] = {
   0,  1,  4,  16, 20, 17, 5,  2,  8,  32, 21, 6,  18, 24, 9,  33, 36, 3,  12, 48, 22, 25,
   37, 40, 34, 10, 7,  19, 28, 13, 49, 52, 41, 38, 26, 23, 29, 53, 11, 35, 44, 14, 50, 56,
   42, 27, 39, 45, 30, 54, 57, 60, 51, 15, 43, 46, 58, 61, 55, 31, 62, 59, 47, 63
 };
-static __constant__ uint8_t kPerm2d[16] = { 0, 1, 4, 5, 2, 8, 6, 9, 3, 12, 10, 7, 13, 11, 14, 15 };
+static __constant__ constexpr uint8_t kPerm2d[16] = { 0, 1, 4, 5, 2, 8, 6, 9, 3, 12, 10, 7, 13, 11, 14, 15 };
 
 __device__ __forceinline__ int perm(int nd, int i)
 {

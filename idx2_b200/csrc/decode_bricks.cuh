@@ -148,15 +148,6 @@ __device__ __forceinline__ int32_t from_negabinary(uint32_t u)
   return (int32_t)((u ^ 0xaaaaaaaau) - 0xaaaaaaaau);
 }
 
-// Coefficient j of a 3D block is the sample kSeq3[j] = x + 4y + 16z (Core/Zfp.h:419 Perm3); of
-// a 2D block kSeq2[j] = u + 4v (Core/Zfp.h:498 Perm2).
-__device__ constexpr uint8_t kSeq3[64] = {
-  0,  1,  4,  16, 20, 17, 5,  2,  8,  32, 21, 6,  18, 24, 9,  33, 36, 3,  12, 48, 22, 25,
-  37, 40, 34, 10, 7,  19, 28, 13, 49, 52, 41, 38, 26, 23, 29, 53, 11, 35, 44, 14, 50, 56,
-  42, 27, 39, 45, 30, 54, 57, 60, 51, 15, 43, 46, 58, 61, 55, 31, 62, 59, 47, 63
-};
-__device__ constexpr uint8_t kSeq2[16] = { 0, 1, 4, 5, 2, 8, 6, 9, 3, 12, 10, 7, 13, 11, 14, 15 };
-
 // Coefficients of a 3D block from planes [first, first + count) of its row of plane words,
 // count <= N: plane first + k becomes bit `top - k` of the coefficients' words. q in sample order.
 template <int N>
@@ -198,8 +189,8 @@ __device__ __forceinline__ void block_words(const unsigned long long* row, int f
       a >>= 31 - top;
       b >>= 31 - top;
     }
-    q[kSeq3[j]] = from_negabinary(a);
-    q[kSeq3[j + 32]] = from_negabinary(b);
+    q[dev::kPerm3d[j]] = from_negabinary(a);
+    q[dev::kPerm3d[j + 32]] = from_negabinary(b);
   }
 }
 
@@ -318,7 +309,7 @@ __device__ __forceinline__ void rebuild_face(const dec_args& a, brick_smem<W>& s
       int32_t q[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        q[kSeq2[j]] = from_negabinary(h[j]);
+        q[dev::kPerm2d[j]] = from_negabinary(h[j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         ilift4_w(q[i], q[i + 4], q[i + 8], q[i + 12]);
@@ -337,7 +328,7 @@ __device__ __forceinline__ void rebuild_face(const dec_args& a, brick_smem<W>& s
     for (int j = 0; j < 16; ++j)
     {
       const unsigned long long u = ((unsigned long long)h[j] << 32) | l[j];
-      q[kSeq2[j]] = (long long)((u ^ dev::kNegaMask) - dev::kNegaMask);
+      q[dev::kPerm2d[j]] = (long long)((u ^ dev::kNegaMask) - dev::kNegaMask);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)

@@ -600,18 +600,11 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, Pu
 constexpr int kRingWords = 16;
 constexpr unsigned kRingMask = (kRingWords - 1) * 128;  // byte offset of a ring word, 32 lanes wide
 
-
-// shifts that give 0 from 32 bits on
+// a shift that gives 0 from 32 bits on
 __device__ __forceinline__ uint32_t shl_to0(uint32_t x, int n)
 {
   uint32_t r;
   asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
-  return r;
-}
-__device__ __forceinline__ uint32_t shr_to0(uint32_t x, int n)
-{
-  uint32_t r;
-  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
   return r;
 }
 
@@ -875,8 +868,9 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 4) k_decode_planes_ring(cons
 }
 
 template <bool WIDE, bool MULTI = false>
-__global__ void __launch_bounds__(kPlaneWarps * 32, WIDE ? 2 : (MULTI ? 6 : 4)) k_decode_planes(const dec1_args a)
+__global__ void __launch_bounds__(kPlaneWarps * 32, WIDE ? 2 : 6) k_decode_planes(const dec1_args a)
 {
+  static_assert(WIDE || MULTI, "units of up to 32 channels, one plane per key: k_decode_planes_ring");
   __shared__ plane_smem sm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ufirst = WIDE ? 0 : a.unit_first;

@@ -158,7 +158,7 @@ struct enc_smem_t
   unsigned alloc, hdr;
   enc_field fp;  // parameters of the current brick's field
   dev::lift_stack stack;
-  int usual_lattice;  // the stack's sweeps from the second level on are lattice_forward's
+  int usual_lattice;  // the stack's sweeps from the second level on are lattice_level's
   double red[2][W];
   int kmin, kmax;
   unsigned long long region;
