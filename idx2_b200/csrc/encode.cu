@@ -713,7 +713,8 @@ __device__ __forceinline__ void code_subband(const enc_args& a, enc_smem_t<NT>& 
     uint32_t* sw = words + 2 + ((2u * (unsigned)nb + 3u) >> 2);
     for (int t = tid; t < nkeys; t += NT)
       sw[t] = (sm.key_bits[t] + 7) / 8;
-    for (int idx = tid; idx < P * kMaxBlocksPerSubband; idx += NT)
+    // (no channel, so no plane: nothing coded, or a refused window, whose keys have no place here)
+    for (int idx = tid; nkeys && idx < P * kMaxBlocksPerSubband; idx += NT)
     {
       const int b = idx & (kMaxBlocksPerSubband - 1), kk = idx / kMaxBlocksPerSubband;
       if (b >= nb || kk >= sm.np[b])
