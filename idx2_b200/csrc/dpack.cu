@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_ranks(const dpack_args a)
     const bool any = a.seg_kmax[si] >= K0;
     if (any && a.seg_kmax[si] - K0 + 1 > kSegKeys)
     {
+      __syncthreads();  // every thread has read the range, and takes this branch
       if (tid == 0)
         a.seg_kmin[si] = 0x7fffffff;  // (the error flag is set: the host packs)
       continue;

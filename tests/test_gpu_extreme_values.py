@@ -50,3 +50,18 @@ def test_values_that_are_no_numbers_match_oracle(idx2g, tmp_path, dtype, value, 
         assert oracle_encode(str(d / "in.raw"), DIMS, dtype, 1, tol, str(d / "o"))[0] == 0
         idx2g.encode(f, out_dir=str(d / "g"), name="kat", field_name="f", num_levels=1, tolerance=tol)
         assert compare_dirs(str(d / "o" / "kat"), str(d / "g" / "kat")) == [], tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-3, 1e100, 1e300])
+def test_bricks_far_apart_match_oracle(idx2g, tmp_path, scale):
+    """Bricks whose exponents lie up to 1,000 apart: from 256 channel keys in a chunk on, more than the
+    device packer's window, the host packs."""
+    f = _base()
+    f[:32, :32, :32] *= scale
+    f[32:, 32:, 32:] *= scale ** 0.5
+    f.tofile(str(tmp_path / "in.raw"))
+    assert oracle_encode(str(tmp_path / "in.raw"), DIMS, "float64", 1, 1e-3, str(tmp_path / "o"))[0] == 0
+    for i in range(3):
+        idx2g.encode(f, out_dir=str(tmp_path / f"g{i}"), name="kat", field_name="f", num_levels=1, tolerance=1e-3)
+        assert compare_dirs(str(tmp_path / "o" / "kat"), str(tmp_path / f"g{i}" / "kat")) == []
