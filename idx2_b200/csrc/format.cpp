@@ -586,7 +586,7 @@ std::string meta_text(const dataset_format& f, const params& p)
 {
   // Core/idx2Common.cpp:150 WriteMetaFile
   std::string o;
-  char buf[512];
+  char buf[1024];  // (the longest line: two values of a sign, 309 digits, a point and 20 decimals)
   o += "(\n";
   o += "  (common\n";
   o += "    (type \"Simulation\")\n";
