@@ -29,8 +29,8 @@
 // Kept bricks are stored x fastest, 33^3 doubles, in natural order.
 //
 // Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
-// 28.3 ms with k_decode_level, 6.2 ms now; one brick per CTA (8 bricks) 184 and 54 us. At
-// 512^3 57 K warp instructions per brick (354 K before), 26% issue activity: what is left is
+// 28.3 ms with k_decode_level, 6.2 ms now; one brick per CTA (8 bricks) 184 and 54 us. At level 0
+// of 512^3 56 K warp instructions per brick (354 K before), 29% issue activity: what is left is
 // latency at 16 warps per SM (128 registers a thread, 99 KB of shared memory per CTA). Not kept,
 // as no faster: the next brick's parameters, exponents and tables fetched ahead (13% slower: more
 // of the slots leave L2), plane words as 32-byte loads or marked evict-first, the next task's

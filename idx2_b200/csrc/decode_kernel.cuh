@@ -594,8 +594,9 @@ __device__ __forceinline__ plane_unit prep_unit(const dec1_args& a, int unit, Pu
 // Measured on one B200 (gpu__time_duration): the three levels of a 1024^3 float32 field at 1e-3
 // 6.65 ms against 9.5 ms with 64-bit windows refilled from global memory where they ran out; 64
 // units, where only the chain counts, 104 against 350 us (145 with the bit scan alone, 124 with
-// the table and the bit scan on different sides of a branch). What bounds it is instructions: 158 K
-// per brick at 74% issue activity, 9 of 32 lanes active, as every step waits for its longest plane.
+// the table and the bit scan on different sides of a branch). What bounds it is instructions: 161 K
+// per brick at 79% issue activity at level 0 of 512^3, 11.5 of 32 lanes active, as every step waits
+// for its longest plane.
 // ---------------------------------------------------------------------------
 constexpr int kRingWords = 16;
 constexpr unsigned kRingMask = (kRingWords - 1) * 128;  // byte offset of a ring word, 32 lanes wide
